@@ -69,7 +69,7 @@ constexpr int DEFAULT_BAND = 8;
 // Pairwise coprime moduli <= 256, largest first (256 = 2^8 and odd numbers
 // with disjoint prime factors), and per modulus the constants of the GEMM
 // epilogue's reduction (2^16 mod p, floor(2^32 / p), a bias) and of the
-// residue pass (2^27 mod p and 1/p in FP64).
+// residue pass (1/p in FP64).
 constexpr int kModList[MAXMOD] = {256, 255, 253, 251, 247, 241, 239, 233, 229,
                                   227, 223, 217, 211, 199, 197, 193, 191, 181};
 static_assert(kModList[0] == 256, "the residue pass takes modulus 0 as the byte of the integer");
@@ -78,7 +78,6 @@ struct ModConst {
     int p, c16;          // p, 2^16 mod p
     unsigned int mrec;   // floor(2^32 / p): floor(y mrec / 2^32) is floor(y / p) or one less (y < 2^28)
     int bias;            // a multiple of p above 2^15 * 255 (keeps the epilogue's sums >= 0)
-    double c27;      // 2^27 mod p (the residue pass, in FP64)
     double inv;      // 1 / p rounded to double
 };
 
@@ -88,7 +87,6 @@ constexpr ModConst make_mod(int p)
                     (int) ((1LL << 16) % p),
                     (unsigned int) ((1ULL << 32) / (unsigned long long) p),
                     (int) (((8650752LL + p - 1) / p) * p),   // a multiple of p >= 2^23 + 2^18
-                    (double) ((1LL << 27) % p),
                     1.0 / (double) p};
 }
 
@@ -198,25 +196,33 @@ double log2_modprod(int nmod)
 
 // ------------------------------------------------------------------ residues
 // The residues of the row / column integers a' = rint(a 2^(P - E)) (|a'| <=
-// 2^53), as signed bytes in [-(p-1)/2, (p-1)/2] (p odd) and [-128, 127]
-// (p = 256).  a' = h 2^27 + l with |h|, |l| <= 2^26 (h by rounding with
-// 1.5 2^52 added), then per odd modulus yb = h (2^27 mod p) + l + 1.5 2^52
-// (one FMA, exact: |y| < 2^35) and q = the nearest integer to y / p, from
-// y = yb - 1.5 2^52 and one FMA with 1.5 2^52 added (y (1/p) is within 2^-23
-// of y / p, which is never closer than 1 / (2p) to a half-integer for odd p).
-// The low words of yb and of that FMA are y and q modulo 2^32 (the low bits of
-// x + 1.5 2^52 are the integer x in two's complement), and r = y - q p is
-// small, so it is one 32-bit integer multiply-add modulo 2^32: three FP64
-// operations and one on the integer pipe per modulus (five FP64 operations
-// when r was formed in FP64: 119 -> 99 us per 4000 x 4000 operand).  For
-// p = 256 the byte is the low byte of l (a' = l mod 256).  Every value is the
-// unique representative of a' mod p in that range, so the bytes equal the
-// integer formulation's.
+// 2^P, P <= 53), as signed bytes congruent to a' mod p.  Per element, a' is
+// formed once as an exact double and as its low 32 bits:
+//   t = a 2^(P - E);  H = the integer nearest to t 2^-32 (1.5 2^52 added),
+//   s = t - H 2^32 (exact, |s| <= 2^31),  sm = s + 1.5 2^52 (rounds s to the
+//   nearest integer, ties to even: H 2^32 is even, so the tie is t's tie too),
+//   a' = H 2^32 + (sm - 1.5 2^52), exact, and its low word is that of sm.
+// Per odd modulus: qm = fma(a', RN(1/p), 1.5 2^52), whose low word is the
+// quotient q modulo 2^32, and r = lo(a') - q p, one 32-bit multiply-add, of
+// which the low byte is stored: one FP64 operation and one integer one per
+// residue.  RN(1/p) is off by at most 2^-53 / p, so a' RN(1/p) is within
+// 2^(P-53) / p of a' / p and |r| <= (p - 1)/2 + 1/2 + 2^(P-53): the centred
+// representative for P <= 51, at most one more for P = 52, 53, which the byte
+// holds for p <= 253.  For p = 255 the reciprocal is within 2^-56 / p and r is
+// centred for every P.  The GEMM's sums stay exact with |r| <= 128, and its
+// epilogue reduces them to [0, p), so C's residues do not depend on which
+// representative was stored.  (The form before this one reduced h 2^27 + l
+// with three FP64 operations per residue: 376-387 us per 8000 x 8000 operand, now
+// 307-311; a 1048576 x 512 operand, 16 moduli: 3.12 -> 2.57 ms, 5.0 TB/s.  Three
+// blocks per SM instead of two are 3 % faster at 2048 x 2048 and 10 % slower at
+// 8000 x 8000.)
+// For p = 256 the byte is the low byte of a'.
 // NM: the modulus count, a template argument so that the modulus loop unrolls
 // (the constants become immediate operands and consecutive moduli interleave).
 template <int NM>
 struct ResidueWriter {
     static constexpr int kMinBlocks = 2;
+    static constexpr bool kResidues = true;
     static __device__ __forceinline__ void write16(const SliceDesc &d, unsigned char *__restrict__ work,
                                                    const unsigned long long *__restrict__ mwork,
                                                    int gr, int gl, const double (&x)[16])
@@ -228,15 +234,17 @@ struct ResidueWriter {
         if (gl == 0 && gr < d.rows)
             reinterpret_cast<int *>(work)[d.e_off + gr] = (fin && mr) ? E + EXP_BIAS : 0;
         const int sh = d.p_bits - E;
-        const double up1 = ldexp(1.0, sh / 2), up2 = ldexp(1.0, sh - sh / 2);
+        const double up1 = pow2(sh / 2), up2 = pow2(sh - sh / 2);
         constexpr double MAGIC = 6755399441055744.0;          // 1.5 2^52
-        double hh[16], lm[16];
+        double av[16];
+        unsigned int lo[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-            const double a = rint((fin ? x[j] : 0.0) * up1 * up2);
-            const double h = (a * 0x1p-27 + MAGIC) - MAGIC;   // nearest integer, |h| <= 2^26
-            hh[j] = h;
-            lm[j] = fma(-h, 0x1p27, a) + MAGIC;              // l + 1.5 2^52, exact
+            const double t = (fin ? x[j] : 0.0) * up1 * up2;
+            const double H = fma(t, 0x1p-32, MAGIC) - MAGIC;
+            const double sm = fma(-H, 0x1p32, t) + MAGIC;
+            av[j] = fma(H, 0x1p32, sm - MAGIC);
+            lo[j] = (unsigned int) __double2loint(sm);
         }
         const int rt = gr / d.tile_rows, rr = gr % d.tile_rows;
         const int kb = gl >> 7, chunk = (gl & 127) >> 4;
@@ -248,23 +256,22 @@ struct ResidueWriter {
             unsigned int r[16];
             if (t == 0) {
 #pragma unroll
-                for (int j = 0; j < 16; ++j) r[j] = (unsigned int) __double2loint(lm[j]);
+                for (int j = 0; j < 16; ++j) r[j] = lo[j];
             } else {
-                const double c27 = kMod.m[t].c27, inv = kMod.m[t].inv;
+                const double inv = kMod.m[t].inv;
                 const unsigned int p = (unsigned int) kMod.m[t].p;
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
-                    const double yb = fma(hh[j], c27, lm[j]);      // y + 1.5 2^52
-                    const double qm = fma(yb - MAGIC, inv, MAGIC);  // q + 1.5 2^52
-                    r[j] = (unsigned int) __double2loint(yb) - (unsigned int) __double2loint(qm) * p;
+                    const double qm = fma(av[j], inv, MAGIC);       // q + 1.5 2^52
+                    r[j] = lo[j] - (unsigned int) __double2loint(qm) * p;
                 }
             }
             uint32_t out[4];
 #pragma unroll
             for (int w = 0; w < 4; ++w) {
-                const uint32_t lo = __byte_perm(r[4 * w], r[4 * w + 1], 0x7740);
-                const uint32_t hi = __byte_perm(r[4 * w + 2], r[4 * w + 3], 0x7740);
-                out[w] = __byte_perm(lo, hi, 0x5410);
+                const uint32_t l2 = __byte_perm(r[4 * w], r[4 * w + 1], 0x7740);
+                const uint32_t h2 = __byte_perm(r[4 * w + 2], r[4 * w + 3], 0x7740);
+                out[w] = __byte_perm(l2, h2, 0x5410);
             }
             *reinterpret_cast<uint4 *>(dst + (long long) t * d.t_stride) =
                 make_uint4(out[0], out[1], out[2], out[3]);

@@ -40,11 +40,19 @@ constexpr int SHAPE_KC = 1, SHAPE_RC = 2;
 // KC (k contiguous): exponent items of 8 rows x 512 k (a warp reads 4 KB of one
 // row), slicing tiles of 16 rows x 256 k (a thread reads its own 16 k).
 // RC (rows contiguous): exponent tiles of 64 rows x 64 k, slicing tiles of
-// 128 rows x 32 k (one k-block) transposed through shared memory.
+// rc_rows x rc_k elements transposed through shared memory.
 // Long contiguous runs per warp matter on B200: 512-byte row pieces 8 MB apart
 // read at half the rate of 4 KB runs.
 constexpr int KC_XR = 8, KC_XK = 512, KC_SR = 16, KC_SK = 256;
-constexpr int RC_SR = 128, RC_SK = 32;
+// RC slicing tile: the slices' k block is 32 bytes, so a 128 x 32 tile writes
+// whole runs of it (128 rows x 32 bytes); the residues' is 128 bytes, of which a
+// 64 x 64 tile writes half a row at a time and a 128 x 32 one a quarter.  Per
+// 8000 x 8000 operand (15 moduli): 360 us at 128 x 32, 307 at 64 x 64, 299 at
+// 32 x 128, whose 256-byte column pieces read slower where the operand is small
+// (256 uneven operands: 0.518, 0.512, 0.534 ms).  The slices at 4000 x 4000:
+// 41.4, 43.0, 47.7 us.
+__host__ __device__ constexpr int rc_rows(bool residues) { return residues ? 64 : 128; }
+__host__ __device__ constexpr int rc_k(bool residues) { return residues ? 64 : 32; }
 
 __host__ __device__ inline int exp_items_of(const SliceDesc &d)
 {
@@ -57,7 +65,8 @@ __host__ __device__ inline int slice_tiles_of(const SliceDesc &d)
 {
     if (d.rows <= 0 || d.kz <= 0) return 0;
     if (d.shape == SHAPE_KC) return ((d.rows_pad + KC_SR - 1) / KC_SR) * ((d.kpad + KC_SK - 1) / KC_SK);
-    return ((d.rows_pad + RC_SR - 1) / RC_SR) * ((d.kpad + RC_SK - 1) / RC_SK);
+    const int sr = rc_rows(d.nmod > 0), sk = rc_k(d.nmod > 0);
+    return ((d.rows_pad + sr - 1) / sr) * ((d.kpad + sk - 1) / sk);
 }
 
 // Which numbering a search runs over: exponent items, KC or RC slicing tiles.
@@ -217,7 +226,8 @@ oz_exp_kernel(const double *__restrict__ src, const SliceDesc *__restrict__ desc
 // included: they hold zero digits).  W::write16 turns one row's 16
 // consecutive k elements into the operand bytes of the GEMM that follows
 // (INT8 slices, or residues modulo the moduli of the modular scheme);
-// W::kMinBlocks is the occupancy the kernel is compiled for.
+// W::kMinBlocks is the occupancy the kernel is compiled for, W::kResidues says
+// which of the two it writes.
 //
 // KC: 16 rows x 256 k per tile.  Warp w loads rows 2w and 2w + 1 with
 // coalesced 16-byte loads (512 contiguous bytes per instruction), the tile is
@@ -294,28 +304,34 @@ slice_rc_kernel(const double *__restrict__ src, const SliceDesc *__restrict__ de
                    int total_tiles, unsigned char *__restrict__ work,
                    const unsigned long long *__restrict__ mwork)
 {
-    __shared__ __align__(16) double tl[RC_SK][RC_SR];
+    // NCH 16-k chunks per tile row, RW rows per warp; each chunk's 16 columns are
+    // RW doubles further on than their pitch alone, so that the lanes of a warp
+    // (RW rows x NCH chunks) read 32 consecutive doubles
+    constexpr int SR = rc_rows(W::kResidues), SK = rc_k(W::kResidues), NCH = SK / 16, RW = 32 / NCH;
+    static_assert(SR * SK == 4096 && SR == 8 * RW, "256 threads, 16 elements each");
+    __shared__ __align__(16) double tl[SK * SR + (NCH - 1) * RW];
     __shared__ int sbeg[DESC_CACHE];
     const DescFinder find = make_finder(sbeg, descs, ndesc, SHAPE_RC);
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
         const SliceDesc &d = descs[find(descs, ndesc, tile, SHAPE_RC)];
         const int local = tile - d.rc_begin;
-        // 128 rows x 32 k; thread (row pair tid % 64, k column tid / 64 + 4 i)
-        // loads 16 bytes of a column, the tile is transposed through shared memory
-        const int ntr = (d.rows_pad + RC_SR - 1) / RC_SR;
-        const int r0 = (local % ntr) * RC_SR, l0 = (local / ntr) * RC_SK;
-        const int rp = threadIdx.x & 63, cg = threadIdx.x >> 6;
+        // thread (row pair rp, k column cg + CG i) loads 16 bytes of a column,
+        // the tile is transposed through shared memory
+        const int ntr = (d.rows_pad + SR - 1) / SR;
+        const int r0 = (local % ntr) * SR, l0 = (local / ntr) * SK;
+        constexpr int RP = SR / 2, CG = 256 / RP;
+        const int rp = threadIdx.x % RP, cg = threadIdx.x / RP;
         const double *base = slice_src(src, d.src_off) + r0 + (long long) l0 * d.ls;
         const int rn = d.rows - r0, ln = d.kz - l0;
         double2 v[8];
-        if (!(reinterpret_cast<uintptr_t>(base) & 15) && !(d.ls & 1) && rn >= RC_SR && ln >= RC_SK) {
+        if (!(reinterpret_cast<uintptr_t>(base) & 15) && !(d.ls & 1) && rn >= SR && ln >= SK) {
 #pragma unroll
             for (int i = 0; i < 8; ++i)
-                v[i] = __ldg(reinterpret_cast<const double2 *>(base + (long long) (cg + 4 * i) * d.ls) + rp);
+                v[i] = __ldg(reinterpret_cast<const double2 *>(base + (long long) (cg + CG * i) * d.ls) + rp);
         } else {
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                const int l = cg + 4 * i;
+                const int l = cg + CG * i;
                 const double *c = base + (long long) l * d.ls + 2 * rp;
                 v[i].x = (l < ln && 2 * rp < rn) ? __ldg(c) : 0.0;
                 v[i].y = (l < ln && 2 * rp + 1 < rn) ? __ldg(c + 1) : 0.0;
@@ -323,16 +339,19 @@ slice_rc_kernel(const double *__restrict__ src, const SliceDesc *__restrict__ de
         }
         __syncthreads();                             // tl of the previous tile is read
 #pragma unroll
-        for (int i = 0; i < 8; ++i) reinterpret_cast<double2 *>(&tl[cg + 4 * i][0])[rp] = v[i];
+        for (int i = 0; i < 8; ++i) {
+            const int l = cg + CG * i;
+            reinterpret_cast<double2 *>(&tl[l * SR + (l >> 4) * RW])[rp] = v[i];
+        }
         __syncthreads();
-        // warp w: rows 16 w .. 16 w + 15, both 16-k chunks (lane: row lane / 2,
-        // chunk lane % 2): each slice's stores from a warp cover 512 contiguous bytes
-        const int r = 16 * (threadIdx.x >> 5) + ((threadIdx.x & 31) >> 1), c = (threadIdx.x & 1) * 16;
+        // lane (row lane / NCH, 16-k chunk lane % NCH) of the warp's RW rows
+        const int lane = threadIdx.x & 31;
+        const int r = RW * (threadIdx.x >> 5) + lane / NCH, c = (lane % NCH) * 16;
         const int gr = r0 + r, gl = l0 + c;
         if (gr >= d.rows_pad || gl >= d.kpad) continue;
         double x[16];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) x[j] = tl[c + j][r];
+        for (int j = 0; j < 16; ++j) x[j] = tl[(c + j) * SR + (c >> 4) * RW + r];
         W::write16(d, work, mwork, gr, gl, x);
     }
 }
