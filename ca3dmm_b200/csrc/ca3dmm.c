@@ -34,6 +34,10 @@
 #define ALIGN_BYTES 256
 #define CANARY_BYTES 256
 #define CANARY_BYTE 0xA5
+/* the device status words, then the k segments' counters (cut tiles: at most one
+ * per CTA boundary and half tile) */
+#define STATUS_WORDS_BYTES 64
+#define STATUS_BYTES (STATUS_WORDS_BYTES + 2 * CA3DMM_DGEMM_SEG_CTAS * (int) sizeof(int))
 
 typedef struct {
     int tk, tm, tn;        /* task ids */
@@ -81,6 +85,12 @@ typedef struct {
     int a_kmajor;                 /* plain mode: transposed A blocks read in place, K-major */
     int plain_merged;             /* plain mode: the kp slabs run as one GEMM over all of k */
     int merge_allowed;            /* CA3DMM_PLAIN_MERGE_SLABS (default 1) */
+    /* plain mode, C of few enough tiles: one product over all of k run as k
+     * segments shared out evenly over the SMs (seg_plan), its operand blocks
+     * whole (wA, wB), its cut tiles' partials in the slab region */
+    int seg_plan, nseg, seg_grid, seg_begin[CA3DMM_DGEMM_SEG_CTAS + 1];
+    size_t off_seg, seg_bytes;
+    blk_t wA, wB;
     /* dst_C block */
     int has_dst, dst_srow, dst_nrow, dst_scol, dst_ncol;
     cudaEvent_t ev[5];
@@ -212,7 +222,7 @@ static void plan_layout(ca3dmm_engine_p e, plan_t *pl)
 {
     size_t off = 0;
     pl->ncanary = 0;
-    pl->off_status = off; off = align_up(off + 64);
+    pl->off_status = off; off = align_up(off + STATUS_BYTES);
     pl->off_packA = off; off = align_up(off + sizeof(ca3dmm_pack_desc_t) * pl->nA);
     pl->off_packB = off; off = align_up(off + sizeof(ca3dmm_pack_desc_t) * pl->nB);
     pl->off_copy = off; off = align_up(off + sizeof(ca3dmm_pack_desc_t));
@@ -224,6 +234,12 @@ static void plan_layout(ca3dmm_engine_p e, plan_t *pl)
     pl->off_ozplan = off; off = align_up(off + pl->oz_plan_bytes);
     pl->crt_plan_bytes = ca3dmm_crt_plan_bytes(2 * pl->crt_nsl, pl->crt_nsl);
     pl->off_crtplan = off; off = align_up(off + pl->crt_plan_bytes);
+    pl->seg_bytes = 0;
+    if (pl->seg_plan) {
+        const size_t mx = (size_t) ca3dmm_dgemm_segments_max(e->m, e->n, e->k);
+        pl->seg_bytes = 2 * mx * sizeof(ca3dmm_dgemm_seg_t);   /* in tile and in list order */
+    }
+    pl->off_seg = off; off = align_up(off + pl->seg_bytes);
     GUARD_BAND(off);
     size_t packs = 0;
     pl->off_A = off;
@@ -249,7 +265,10 @@ static void plan_layout(ca3dmm_engine_p e, plan_t *pl)
     pl->off_slab = off;
     int nslab = e->kp * pl->ksplit;          /* plain mode's sub-slabs; split mode uses kp of them */
     if (pl->crt_nsl > nslab) nslab = pl->crt_nsl;
-    if (nslab > 1) off = align_up(off + sizeof(double) * pl->slab_stride * (size_t) nslab);
+    if (pl->seg_plan && e->gemm_mode == CA3DMM_GEMM_PLAIN)
+        off = align_up(off + ca3dmm_dgemm_segments_ws_bytes(e->m, e->n, e->k));
+    else if (nslab > 1)
+        off = align_up(off + sizeof(double) * pl->slab_stride * (size_t) nslab);
     GUARD_BAND(off);
     pl->off_cout = off;
     off = align_up(off + sizeof(double) * (size_t) e->m * (size_t) e->n);
@@ -371,10 +390,16 @@ static int plan_build(ca3dmm_engine_p e)
     pl->groups = (group_t *) calloc((size_t) pl->ngroup, sizeof(group_t));
     pl->A = (blk_t *) calloc((size_t) pl->nA, sizeof(blk_t));
     pl->B = (blk_t *) calloc((size_t) pl->nB, sizeof(blk_t));
-    pl->ksplit = choose_ksplit(e, pl->sym);
     int merge;
     GET_ENV_INT_VAR(merge, "CA3DMM_PLAIN_MERGE_SLABS", "plain_merge_slabs", 1, 0, 1);
     pl->merge_allowed = merge;
+    /* k segments instead of kp slabs and their sub-slabs, where one product over
+     * all of k may take their place (B^T B keeps its slabs: the host-buffer exec
+     * is pipelined over them, and with its long k the sub-slabs already fill the
+     * rounds to 99 %) */
+    pl->seg_plan = merge && !pl->sym && !e->is_BTB &&
+                   ca3dmm_dgemm_segments_max(e->m, e->n, e->k) > 0;
+    pl->ksplit = pl->seg_plan ? 1 : choose_ksplit(e, pl->sym);
     GET_ENV_INT_VAR(pl->crt_band, "CA3DMM_CRT_BAND", "crt_band", 32, 0, 1 << 20);
     pl->crt_band_env = pl->crt_band;
     GET_ENV_INT_VAR(pl->crt_tile_n, "CA3DMM_CRT_TILE_N", "crt_tile_n", 256, 128, 256);
@@ -449,7 +474,7 @@ static int plan_build(ca3dmm_engine_p e)
         g->m = e->m; g->n = e->n; g->k = kz;
     }
     plan_layout(e, pl);
-    pl->stage_bytes = pl->off_crtplan + pl->crt_plan_bytes;
+    pl->stage_bytes = pl->off_seg + pl->seg_bytes;
     return CA3DMM_OK;
 }
 
@@ -969,9 +994,22 @@ static int plan_upload(ca3dmm_engine_p e, const void *A, int ldA, const void *B,
      * aligned start in place, the others (an odd first k index) copied, not
      * transposed, into the K-major layout. */
     pl->a_kmajor = e->trans_A && (ldA & 1) == 0;
+    /* k segments: one block over all of k on either side (a packed copy takes the
+     * place of the slabs' copies, which are at least as large together) */
+    const int seg = pl->seg_plan && e->gemm_mode == CA3DMM_GEMM_PLAIN;
+    pl->wA = pl->A[0];
+    pl->wA.cols = e->k;
+    pl->wA.kld = ca3dmm_round_up(e->k > 0 ? e->k : 1, 2);
+    pl->wB = pl->B[0];
+    pl->wB.rows = e->k;
+    pl->wB.ld = ca3dmm_round_up(e->k > 0 ? e->k : 1, 2);
     for (int i = 0; i < pl->nA; i++) {
-        blk_t *b = &pl->A[i];
+        blk_t *b = seg ? &pl->wA : &pl->A[i];
         ca3dmm_pack_desc_t *d = &pa[i];
+        if (seg && i > 0) {
+            memset(d, 0, sizeof(*d));
+            continue;
+        }
         a_pack_desc(e, pl, b, 0, b->rows, ldA, d);
         b->direct = NULL;
         if ((!e->trans_A || pl->a_kmajor) && (ldA & 1) == 0 &&
@@ -990,9 +1028,10 @@ static int plan_upload(ca3dmm_engine_p e, const void *A, int ldA, const void *B,
         pl->pack_tiles_A = ca3dmm_pack_tiles(pa, pl->nA);
     ca3dmm_pack_desc_t *pb = (ca3dmm_pack_desc_t *) (h + pl->off_packB);
     for (int i = 0; i < pl->nB; i++) {
-        blk_t *b = &pl->B[i];
+        blk_t *b = seg ? &pl->wB : &pl->B[i];
         ca3dmm_pack_desc_t *d = &pb[i];
         memset(d, 0, sizeof(*d));
+        if (seg && i > 0) continue;
         d->rows = b->rows; d->cols = b->cols; d->trans = e->trans_B; d->lds = ldB;
         d->src_off = e->trans_B ? (long long) b->c0 + (long long) b->r0 * ldB
                                 : (long long) b->r0 + (long long) b->c0 * ldB;
@@ -1014,8 +1053,8 @@ static int plan_upload(ca3dmm_engine_p e, const void *A, int ldA, const void *B,
      * slabs' blocks, no slab buffers, no slab sum.  The plain path's contract
      * is k u |A||B| accuracy, not the slab sum's rounding order (split
      * precision keeps the slabs: its exponents are per slab). */
-    pl->plain_merged = 0;
-    if (pl->merge_allowed && e->gemm_mode == CA3DMM_GEMM_PLAIN && !pl->sym && !e->is_BTB &&
+    pl->plain_merged = seg;
+    if (!seg && pl->merge_allowed && e->gemm_mode == CA3DMM_GEMM_PLAIN && !pl->sym && !e->is_BTB &&
         pl->ksplit == 1 &&
         e->kp > 1 && pl->tmn == 1 && pl->tnn == 1 && pl->A[0].direct && pl->B[0].direct &&
         (long long) ((e->m + 127) / 128) * ((e->n + 127) / 128) >= 4LL * CA3DMM_SMS_B200) {
@@ -1026,7 +1065,7 @@ static int plan_upload(ca3dmm_engine_p e, const void *A, int ldA, const void *B,
         pl->pack_tiles_A = ca3dmm_pack_tiles(pa, pl->nA);
     }
     pl->packB_tma = 0;
-    if (e->trans_B && !pl->plain_merged && ca3dmm_pack_tma_prepare(pb, pl->nB, (const double *) B, h + pl->off_tmapB,
+    if (e->trans_B && (seg || !pl->plain_merged) && ca3dmm_pack_tma_prepare(pb, pl->nB, (const double *) B, h + pl->off_tmapB,
                                               &pl->pack_tiles_B) == CA3DMM_OK)
         pl->packB_tma = 1;
     else
@@ -1048,7 +1087,7 @@ static int plan_upload(ca3dmm_engine_p e, const void *A, int ldA, const void *B,
 
     for (int i = 0; i < pl->ngroup; i++) {
         group_t *g = &pl->groups[i];
-        const blk_t *ba = &pl->A[g->a_blk], *bb = &pl->B[g->b_blk];
+        const blk_t *ba = seg ? &pl->wA : &pl->A[g->a_blk], *bb = seg ? &pl->wB : &pl->B[g->b_blk];
         const double *a = ba->direct ? ba->direct : (const double *) (w + ba->off);
         const long long lda = ba->direct ? ba->direct_ld : (pl->a_kmajor ? ba->kld : ba->ld);
         const double *b = bb->direct ? bb->direct : (const double *) (w + bb->off);
@@ -1095,6 +1134,18 @@ static int plan_upload(ca3dmm_engine_p e, const void *A, int ldA, const void *B,
     int rc = ca3dmm_dgemm_plan_encode_tn(gd, pl->ngroup * ks, h + pl->off_gemm, &pl->gemm_tiles,
                                          pl->plain_tile_n);
     if (rc) return rc;
+    if (seg) {
+        const int mx = ca3dmm_dgemm_segments_max(e->m, e->n, e->k);
+        ca3dmm_dgemm_seg_t *sg = (ca3dmm_dgemm_seg_t *) (h + pl->off_seg);
+        int *order = (int *) malloc(sizeof(int) * (size_t) mx), ncounter = 0;
+        if (!order) return CA3DMM_ENOMEM;
+        rc = ca3dmm_dgemm_segments(e->m, e->n, e->k, pl->plain_tile_n, sg, order, pl->seg_begin,
+                                   &pl->nseg, &pl->seg_grid, &ncounter);
+        for (int i = 0; !rc && i < pl->nseg; i++) sg[mx + i] = sg[order[i]];
+        free(order);
+        if (!rc && ncounter > 2 * CA3DMM_DGEMM_SEG_CTAS) rc = CA3DMM_EINVAL;
+        if (rc) return rc;
+    }
     if (e->gemm_mode == CA3DMM_GEMM_OZAKI) {
         ca3dmm_oz_blk_t *ob = pl->ob;
         ca3dmm_oz_src_t *os = pl->os;
@@ -1192,7 +1243,7 @@ static int plan_upload(ca3dmm_engine_p e, const void *A, int ldA, const void *B,
         if (rc) return rc;
         e->crt_bits = pl->crt.p_min;
     }
-    memset(h + pl->off_status, 0, 64);
+    memset(h + pl->off_status, 0, STATUS_BYTES);
     CA3DMM_CUDA_TRY(cudaMemcpyAsync(w, h, pl->stage_bytes, cudaMemcpyHostToDevice, st));
     for (int i = 0; i < pl->ncanary; i++)
         CA3DMM_CUDA_TRY(cudaMemsetAsync(w + pl->canary[i], CANARY_BYTE, CANARY_BYTES, st));
@@ -1217,6 +1268,22 @@ static int launch_pack_side(ca3dmm_engine_p e, int which, const void *src, cudaS
                                       (double *) w, (int *) (w + pl->off_status), 5.0, st);
     return ca3dmm_pack_launch((const double *) src, (double *) w,
                               (const ca3dmm_pack_desc_t *) (w + off_desc), nd, tiles, st);
+}
+
+/* The k segments of the plan: all of them by the CTAs' lists, or those of one
+ * range (a band of output rows). */
+static int launch_segments(ca3dmm_engine_p e, const ca3dmm_tile_ranges_t *rg, cudaStream_t st)
+{
+    plan_t *pl = (plan_t *) e->impl;
+    char *w = (char *) e->workbuf_d;
+    const ca3dmm_dgemm_seg_t *sg = (const ca3dmm_dgemm_seg_t *) (w + pl->off_seg);
+    if (!rg) sg += pl->seg_bytes / (2 * sizeof(*sg));
+    const int lo = rg ? rg->begin[0] : 0, hi = rg ? lo + rg->len[0] : pl->nseg;
+    return ca3dmm_dgemm_launch_segments(
+        (const char *) pl->stage + pl->off_gemm, pl->ngroup * pl->ksplit, sg,
+        rg ? NULL : pl->seg_begin, lo, hi, pl->seg_grid, pl->a_kmajor, w + pl->off_slab,
+        (int *) (w + pl->off_status + STATUS_WORDS_BYTES), (int *) (w + pl->off_status), 5.0, st,
+        pl->plain_tile_n);
 }
 
 /* The device status word after a call: 0, a bounded wait that ran out, or
@@ -1333,7 +1400,7 @@ static int exec_device(ca3dmm_engine_p e, const void *src_A, int ldA, const void
         pl->c_ldB != ldB || pl->c_dst != dst_C || pl->c_ldC != ldC) {
         rc = plan_upload(e, src_A, ldA, src_B, ldB, dst_C, ldC, st);
         if (rc) return rc;
-    } else if (cudaMemsetAsync(w + pl->off_status, 0, 64, st) != cudaSuccess) {
+    } else if (cudaMemsetAsync(w + pl->off_status, 0, STATUS_BYTES, st) != cudaSuccess) {
         return CA3DMM_ECUDA;
     }
     int timing = e->sync_exec && pl->events_ok;
@@ -1363,6 +1430,8 @@ static int exec_device(ca3dmm_engine_p e, const void *src_A, int ldA, const void
     } else if (e->gemm_mode == CA3DMM_GEMM_OZAKI) {
         rc = ca3dmm_oz_run_gemm(&pl->oz, status_d, 5.0, st);
         if (!rc) rc = ca3dmm_oz_run_nonfinite(&pl->oz, NULL, src_A, src_B, st);
+    } else if (pl->seg_plan) {
+        rc = launch_segments(e, NULL, st);
     } else
         rc = ca3dmm_dgemm_launch_tn(w + pl->off_gemm, pl->ngroup * pl->ksplit, pl->gemm_tiles,
                                     pl->a_kmajor, status_d, 5.0, st, pl->plain_tile_n);
@@ -1585,7 +1654,9 @@ static int hx_build_bands(ca3dmm_engine_p e, struct host_exec *x, cudaStream_t s
     if (e->is_BTB || !whole || ((ozaki && pl->oz_fused) ? 1 : e->kp) * tnn > CA3DMM_MAX_RANGES ||
         (!ozaki && pl->ksplit > 1))
         return 0;
-    const int raster = e->raster > 0 ? e->raster : 8;
+    /* k segments are numbered in bands of 8 tile rows whatever the raster */
+    const int seg = !ozaki && pl->seg_plan;
+    const int raster = seg || e->raster <= 0 ? 8 : e->raster;
     const int bn = ozaki ? 64 : pl->plain_tile_n;
     /* tile numbering of the GEMM plans: per group (plain) or per unit of
      * (task_m, task_n) with its kp slabs chained (split precision) */
@@ -1629,7 +1700,17 @@ static int hx_build_bands(ca3dmm_engine_p e, struct host_exec *x, cudaStream_t s
             ca3dmm_tile_ranges_t *rg = &x->rng[c];
             memset(rg, 0, sizeof(*rg));
             const int row_lo = r / 128, nrow_t = band_rows / 128;
-            for (int tk = 0; tk < ((chained || (!ozaki && pl->plain_merged)) ? 1 : e->kp); tk++)
+            if (seg) {
+                const ca3dmm_dgemm_seg_t *sg =
+                    (const ca3dmm_dgemm_seg_t *) ((char *) pl->stage + pl->off_seg);
+                int lo = 0, hi;
+                while (lo < pl->nseg && sg[lo].tm < row_lo) lo++;
+                for (hi = lo; hi < pl->nseg && sg[hi].tm < row_lo + nrow_t;) hi++;
+                rg->n = 1;
+                rg->begin[0] = lo;
+                rg->len[0] = hi - lo;
+            }
+            for (int tk = 0; !seg && tk < ((chained || (!ozaki && pl->plain_merged)) ? 1 : e->kp); tk++)
                 for (int tn = 0; tn < tnn; tn++) {
                     const int g = (tk * tmn + tm) * tnn + tn;
                     const group_t *gg = &pl->groups[g];
@@ -1649,7 +1730,7 @@ static int hx_build_bands(ca3dmm_engine_p e, struct host_exec *x, cudaStream_t s
             } else {
                 ca3dmm_pack_desc_t *pd = (ca3dmm_pack_desc_t *) dh;
                 for (int tk = 0; tk < e->kp; tk++) {
-                    const blk_t *b = &pl->A[blocks[tk]];
+                    const blk_t *b = seg ? &pl->wA : &pl->A[blocks[tk]];
                     ca3dmm_pack_desc_t *d = &pd[tk];
                     memset(d, 0, sizeof(*d));
                     /* read in place by the GEMM, or a slab the merged plain GEMM skips */
@@ -1748,7 +1829,7 @@ static int hx_btb_slabs(ca3dmm_engine_p e, struct host_exec *x, const void *B_h,
     }
     char *w = (char *) e->workbuf_d;
     int *status_d = (int *) (w + pl->off_status);
-    CA3DMM_CUDA_TRY(cudaMemsetAsync(status_d, 0, 64, st));
+    CA3DMM_CUDA_TRY(cudaMemsetAsync(status_d, 0, STATUS_BYTES, st));
     /* copies in: B slab by slab */
     for (int j = 0; j < kp; j++) {
         int k0, kz;
@@ -1896,7 +1977,7 @@ static int exec_host(ca3dmm_engine_p e, const void *A_h, int ldA, const void *B_
     }
     char *w = (char *) e->workbuf_d;
     int *status_d = (int *) (w + pl->off_status);
-    CA3DMM_CUDA_TRY(cudaMemsetAsync(status_d, 0, 64, st));
+    CA3DMM_CUDA_TRY(cudaMemsetAsync(status_d, 0, STATUS_BYTES, st));
     /* copies in: all of B, then the op(A) rows band by band */
     rc = hx_copy_in_B(e, x, B_h, ldB);
     if (rc) return rc;
@@ -1934,7 +2015,9 @@ static int exec_host(ca3dmm_engine_p e, const void *A_h, int ldA, const void *B_
         } else {
             rc = ca3dmm_pack_launch(x->dA, (double *) w, (const ca3dmm_pack_desc_t *) dd, x->ndesc,
                                     x->ntile[c][0], st);
-            if (!rc)
+            if (!rc && pl->seg_plan)
+                rc = launch_segments(e, &x->rng[c], st);
+            else if (!rc)
                 rc = ca3dmm_dgemm_launch_ranges_tn(w + pl->off_gemm, pl->ngroup, &x->rng[c],
                                                    pl->a_kmajor, status_d, 5.0, st,
                                                    pl->plain_tile_n);

@@ -78,6 +78,35 @@ int ca3dmm_dgemm_launch_ranges_tn(const void *dev_plan, int nprob,
                                   int *dev_status, double timeout_s, cudaStream_t stream,
                                   int tile_n);
 
+/* ---- k segments -----------------------------------------------------------
+ * One m x n x k product run as k segments of its 128 x 128 tiles, shared out
+ * evenly over the SMs (tiles cut between CTAs are summed in segment order by
+ * the CTA that finishes last).  ca3dmm_dgemm_segments fills the segments in
+ * tile order (tn counts tile_n columns), the CTAs' lists of them and the
+ * number of counters (cut tiles, one zeroed int each; the launch leaves them
+ * zero); segs and order hold ca3dmm_dgemm_segments_max entries, cta_begin 149.
+ * CA3DMM_EINVAL when the product has too many tiles for this form (max 0). */
+#define CA3DMM_DGEMM_CHUNK 16        /* 16-k blocks per accumulation chain */
+#define CA3DMM_DGEMM_SEG_CTAS 148
+typedef struct {
+    int tm, tn;          /* tile */
+    int kt0, kt1;        /* 16-k blocks [kt0, kt1) */
+    int part, nparts;    /* of the tile's segments */
+    int slot0, counter;  /* first partial slot, counter (cut tiles) */
+} ca3dmm_dgemm_seg_t;
+int ca3dmm_dgemm_segments_max(int m, int n, int k);
+size_t ca3dmm_dgemm_segments_ws_bytes(int m, int n, int k);
+int ca3dmm_dgemm_segments(int m, int n, int k, int tile_n, ca3dmm_dgemm_seg_t *segs, int *order,
+                          int *cta_begin, int *nseg, int *grid, int *ncounter);
+/* Problem 0 of an encoded plan (its host copy): dev_segs in the order of the
+ * CTAs' lists over `grid` CTAs (cta_begin, a host array), or (cta_begin NULL) in
+ * tile order, of which the segments [lo, hi) alone run, round robin. */
+int ca3dmm_dgemm_launch_segments(const void *host_plan, int nprob,
+                                 const ca3dmm_dgemm_seg_t *dev_segs, const int *cta_begin, int lo,
+                                 int hi, int grid, int a_kmajor, void *partials, int *counters,
+                                 int *dev_status, double timeout_s, cudaStream_t stream,
+                                 int tile_n);
+
 /* ---- pack / transpose ----------------------------------------------------
  * Batched block copies between column-major matrices.  Descriptor j copies a
  * rows x cols block: dst[r + c*ldd] = trans ? src[c + r*lds] : src[r + c*lds],

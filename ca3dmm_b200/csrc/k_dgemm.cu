@@ -30,7 +30,9 @@
 // disjoint chunk sets, and the C pairs (m, m+1) stay adjacent.
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <atomic>
 #include "k_common.cuh"
@@ -101,24 +103,52 @@ __device__ __forceinline__ void dmma(double (&d)[4], double a0, double a1, doubl
         : "d"(a0), "d"(a1), "d"(b0));
 }
 
-__device__ __forceinline__ void store_pair(const DProb &p, int m, int n, double v0, double v1)
+// Rows m, m + 1 of one column, alpha v + beta C.
+__device__ __forceinline__ void store_pair(double *c, bool two, bool vec, double alpha, double beta,
+                                           double v0, double v1)
 {
-    if (n >= p.n || m >= p.m) return;
-    double *c = p.C + (long long) m + (long long) n * p.ldc;
-    if (p.vec_ok && m + 1 < p.m) {
+    if (vec && two) {
         double2 o;
-        if (p.beta != 0.0) {
+        if (beta != 0.0) {
             double2 old = *reinterpret_cast<const double2 *>(c);
-            o.x = p.alpha * v0 + p.beta * old.x;
-            o.y = p.alpha * v1 + p.beta * old.y;
+            o.x = alpha * v0 + beta * old.x;
+            o.y = alpha * v1 + beta * old.y;
         } else {
-            o.x = p.alpha * v0;
-            o.y = p.alpha * v1;
+            o.x = alpha * v0;
+            o.y = alpha * v1;
         }
         *reinterpret_cast<double2 *>(c) = o;
     } else {
-        c[0] = p.beta != 0.0 ? p.alpha * v0 + p.beta * c[0] : p.alpha * v0;
-        if (m + 1 < p.m) c[1] = p.beta != 0.0 ? p.alpha * v1 + p.beta * c[1] : p.alpha * v1;
+        c[0] = beta != 0.0 ? alpha * v0 + beta * c[0] : alpha * v0;
+        if (two) c[1] = beta != 0.0 ? alpha * v1 + beta * c[1] : alpha * v1;
+    }
+}
+
+// This thread's part of a finished tile: its first row mb, first column nb.
+// The problem's fields are read once into registers: read through the pointer
+// they were loaded again after each of the 32 stores (which may alias them),
+// 6-7 us per tile instead of 2-4.
+template <int MI>
+__device__ __forceinline__ void store_tile(const DProb &prob, int mb, int nb,
+                                           const double (&acc)[MI][4][4])
+{
+    const int m = prob.m, n = prob.n;
+    const bool vec = prob.vec_ok;
+    const double alpha = prob.alpha, beta = prob.beta;
+    const long long ldc = prob.ldc;
+    double *c0 = prob.C + (long long) mb + (long long) nb * ldc;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        if (nb + j >= n) break;
+        double *c = c0 + j * ldc;
+#pragma unroll
+        for (int i = 0; i < MI; ++i) {
+            const int r = mb + 16 * i;
+            if (r >= m) break;
+            store_pair(c + 16 * i, r + 1 < m, vec, alpha, beta,
+                       j < 4 ? acc[i][j & 3][0] : acc[i][j & 3][1],
+                       j < 4 ? acc[i][j & 3][2] : acc[i][j & 3][3]);
+        }
     }
 }
 
@@ -340,13 +370,7 @@ dgemm_dmma_grouped(const CUtensorMap *__restrict__ tmaps, const DProb *__restric
 
         const int mb = tm * BM + wm * 16 * MI + 2 * (AK ? sigma_row(g) : g);
         const int nb = tn * TBN + wn * 32 + 8 * t;
-#pragma unroll
-        for (int i = 0; i < MI; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                store_pair(p, mb + 16 * i, nb + j, acc[i][j][0], acc[i][j][2]);
-                store_pair(p, mb + 16 * i, nb + 4 + j, acc[i][j][1], acc[i][j][3]);
-            }
+        store_tile<MI>(p, mb, nb, acc);
     }
 
     if (producer) {
@@ -366,6 +390,313 @@ dgemm_dmma_grouped(const CUtensorMap *__restrict__ tmaps, const DProb *__restric
     }
 }
 #undef CA3DMM_PB
+
+// ------------------------------------------------------------------ k segments
+// One problem whose tiles do not fill the chip evenly: the work list holds k
+// segments of tiles instead of whole tiles (ca3dmm_dgemm_segments below), and a
+// CTA runs the segments of its list in turn.  A tile cut into several segments
+// is finished by whichever CTA completes its last one: every CTA writes its
+// partial tile to the workspace and counts up the tile's counter, and the one
+// that counts last adds the partials in segment order and stores C.  No CTA
+// ever waits for another, and the order of the sum is fixed.
+//
+// Inside a segment the accumulators restart every `chunk` k tiles: the partial
+// sums move to a running total in TMEM, which this kernel's MMAs leave free
+// (the same thread writes and reads its words, 128 per thread at 128 columns).
+// Rounding errors grow with the length of a chain of additions, so chunks of
+// 256 k keep the result at least as accurate as the k sub-slabs of up to
+// several thousand k, summed by a kernel of their own, that these shapes ran as
+// before.  (All warps at once lost 1.2 us per chunk of 35 us.)
+__device__ __forceinline__ void tmem_ld32_wait(uint32_t taddr, uint32_t (&v)[32])
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
+        "%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+          "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
+          "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]),
+          "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]),
+          "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32])
+{
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
+        "%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]),
+          "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]),
+          "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]),
+          "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]),
+          "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+        : "memory");
+}
+
+// acc of m16 tile i (4 x 4 doubles = 32 words per thread) += its TMEM total
+__device__ __forceinline__ void total_add(uint32_t taddr, double (&acc)[4][4])
+{
+    uint32_t v[32];
+    tmem_ld32_wait(taddr, v);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            acc[j][e] = __hiloint2double((int) v[8 * j + 2 * e + 1], (int) v[8 * j + 2 * e]) + acc[j][e];
+}
+
+__device__ __forceinline__ void total_store(uint32_t taddr, const double (&acc)[4][4])
+{
+    uint32_t v[32];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            v[8 * j + 2 * e] = (uint32_t) __double2loint(acc[j][e]);
+            v[8 * j + 2 * e + 1] = (uint32_t) __double2hiint(acc[j][e]);
+        }
+    tmem_st32(taddr, v);
+}
+
+// Order of a launch: CTA b runs segments begin[b] .. begin[b + 1] - 1 (the
+// balanced lists of a whole problem), or, without lists, segments lo + b,
+// lo + b + grid, ... below hi (a band of output rows).  It travels with the
+// tensor maps and the problem in the launch's parameters, so that a CTA's first
+// copy waits for one load from global memory (its first segment).
+struct SegOrder {
+    int lists, lo, hi;
+    int begin[CA3DMM_DGEMM_SEG_CTAS + 1];
+};
+
+struct SegCursor {
+    int pos, end, step, kt, kt1, m0, n0;
+    bool valid;
+};
+
+template <bool AK, int TBN>
+__global__ void __launch_bounds__(THREADS, 1)
+dgemm_dmma_segments(const __grid_constant__ CUtensorMap map_a,
+                    const __grid_constant__ CUtensorMap map_b, const __grid_constant__ DProb prob,
+                    const __grid_constant__ SegOrder order,
+                    const ca3dmm_dgemm_seg_t *__restrict__ segs, int chunk, double2 *__restrict__ partials, int *__restrict__ counters, int *status,
+                    unsigned long long limit_ns)
+{
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *smem = reinterpret_cast<uint8_t *>(
+        (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    using T = DTile<TBN>;
+    constexpr int STAGES = T::STAGES, STAGE_BYTES = T::STAGE_BYTES, MI = T::MI;
+    constexpr uint32_t TOTAL_COLS = 2 * 32 * MI;      // two warps per TMEM lane quarter
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem + STAGES * STAGE_BYTES);
+    uint64_t *empty = full + STAGES;
+    __shared__ volatile int abort_flag;
+    __shared__ uint64_t fix_bar[2];                   // partial written; the counter's answer
+    __shared__ volatile int last_part;
+    __shared__ uint32_t tmem_slot;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool producer = threadIdx.x == 0;
+    if (producer) {
+        tmap_prefetch(&map_a);
+        tmap_prefetch(&map_b);
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], CONSUMER_WARPS);
+        }
+        mbar_init(&fix_bar[0], CONSUMER_WARPS);
+        mbar_init(&fix_bar[1], 1);
+        abort_flag = 0;
+        fence_barrier_init();
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         smem_u32(&tmem_slot)),
+                     "r"(TOTAL_COLS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t total = tmem_slot + ((uint32_t) ((warp & 3) * 32) << 16) +
+                           (uint32_t) ((warp >> 2) * 32 * MI);
+
+    const int first = order.lists ? order.begin[blockIdx.x] : order.lo + (int) blockIdx.x;
+    const int end = order.lists ? order.begin[blockIdx.x + 1] : order.hi;
+    const int step = order.lists ? 1 : (int) gridDim.x;
+
+    // thread 0's cursor over the loads, in shared memory: in registers every
+    // thread would hold it, and the K-major form spilled
+    __shared__ SegCursor lc;
+    uint32_t issued = 0;
+    auto open_seg = [&]() {
+        lc.valid = lc.pos < end;
+        if (!lc.valid) return;
+        const ca3dmm_dgemm_seg_t &g = segs[lc.pos];
+        lc.kt = g.kt0;
+        lc.kt1 = g.kt1;
+        lc.m0 = g.tm * BM;
+        lc.n0 = g.tn * TBN;
+    };
+    // Issue load number `issued` at the cursor (producer thread only).
+    auto issue_one = [&]() -> bool {
+        if (!lc.valid) return true;
+        const uint32_t s = issued % STAGES, ph = (issued / STAGES) & 1u;
+        if (!mbar_wait_bounded(&empty[s], ph ^ 1u, &abort_flag, status,
+                               CA3DMM_DEV_TIMEOUT_PRODUCE, limit_ns))
+            return false;
+        const CUtensorMap *ta = &map_a, *tb = &map_b;
+        uint8_t *sA = smem + s * STAGE_BYTES;
+        uint8_t *sB = sA + A_BYTES;
+        mbar_arrive_expect_tx(&full[s], STAGE_BYTES);
+        if (AK) {
+            tma_load_2d(sA, ta, lc.kt * BK, lc.m0, &full[s]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < BM / 16; ++j)
+                tma_load_2d(sA + j * 2048, ta, lc.m0 + 16 * j, lc.kt * BK, &full[s]);
+        }
+        tma_load_2d(sB, tb, lc.kt * BK, lc.n0, &full[s]);
+        ++issued;
+        if (++lc.kt >= lc.kt1) {
+            lc.pos += step;
+            open_seg();
+        }
+        return true;
+    };
+    if (producer) {
+        lc.pos = first;
+        open_seg();
+        for (int s = 0; s < STAGES - 1; ++s)
+            if (!issue_one()) break;
+    }
+
+    const int g = lane >> 2, t = lane & 3;
+    const int wm = warp / T::WN, wn = warp % T::WN;
+    uint32_t it = 0;            // loads consumed so far
+    uint32_t nfix = 0;          // partial tiles written so far (phase of fix_bar)
+    double acc[MI][4][4];
+    bool ok = true;
+
+    for (int pos = first; pos < end && ok; pos += step) {
+        const ca3dmm_dgemm_seg_t &sg = segs[pos];
+        int left = sg.kt1 - sg.kt0;
+        // the warps of rows 64 .. 127 start with half a chunk: of an SM quarter's two
+        // warps one keeps the tensor pipe busy while the other moves its sums
+        int len = warp >= CONSUMER_WARPS / 2 ? chunk / 2 : chunk;
+        bool totalled = false;
+        for (;;) {
+#pragma unroll
+            for (int i = 0; i < MI; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.0;
+            const int now = min(left, len);
+            len = chunk;
+            ok = k_loop<AK, TBN>(smem, full, empty, now, it, acc, &abort_flag, status, limit_ns,
+                                 producer, issue_one, wm, wn, g, t, lane);
+            if (!ok) break;
+            left -= now;
+            if (totalled) {
+#pragma unroll
+                for (int i = 0; i < MI; ++i) total_add(total + 32 * i, acc[i]);
+            }
+            if (left <= 0) break;
+#pragma unroll
+            for (int i = 0; i < MI; ++i) total_store(total + 32 * i, acc[i]);
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            totalled = true;
+        }
+        if (!ok) break;
+
+        const int nparts = sg.nparts;
+        if (nparts > 1) {
+            // words of a partial tile: (m16 tile, n8 tile, row half) outermost, then the thread
+            constexpr int PART = MI * 8 * THREADS;           // double2 of one partial tile
+            double2 *mine = partials + (long long) (sg.slot0 + sg.part) * PART + threadIdx.x;
+#pragma unroll
+            for (int i = 0; i < MI; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    __stcg(mine + (i * 8 + j * 2) * THREADS, make_double2(acc[i][j][0], acc[i][j][1]));
+                    __stcg(mine + (i * 8 + j * 2 + 1) * THREADS,
+                           make_double2(acc[i][j][2], acc[i][j][3]));
+                }
+            __threadfence();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&fix_bar[0]);
+            const uint32_t ph = nfix & 1u;
+            ++nfix;
+            if (producer) {
+                if (!mbar_wait_bounded(&fix_bar[0], ph, &abort_flag, status,
+                                       CA3DMM_DEV_TIMEOUT_ACCUM, limit_ns)) {
+                    ok = false;
+                } else {
+                    const bool last = atomicAdd(counters + sg.counter, 1) == nparts - 1;
+                    if (last) counters[sg.counter] = 0;      // for the next launch
+                    __threadfence();
+                    last_part = last;
+                    mbar_arrive(&fix_bar[1]);
+                }
+            }
+            ok = ok && mbar_wait_bounded(&fix_bar[1], ph, &abort_flag, status,
+                                         CA3DMM_DEV_TIMEOUT_ACCUM, limit_ns);
+            if (!ok) break;
+            if (!last_part) continue;
+            __threadfence();
+            const double2 *part = partials + (long long) sg.slot0 * PART + threadIdx.x;
+#pragma unroll
+            for (int i = 0; i < MI; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const double2 lo = __ldcg(part + (i * 8 + j * 2) * THREADS);
+                    const double2 hi = __ldcg(part + (i * 8 + j * 2 + 1) * THREADS);
+                    acc[i][j][0] = lo.x; acc[i][j][1] = lo.y;
+                    acc[i][j][2] = hi.x; acc[i][j][3] = hi.y;
+                }
+            for (int q = 1; q < nparts; ++q) {
+                part += PART;
+#pragma unroll
+                for (int i = 0; i < MI; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const double2 lo = __ldcg(part + (i * 8 + j * 2) * THREADS);
+                        const double2 hi = __ldcg(part + (i * 8 + j * 2 + 1) * THREADS);
+                        acc[i][j][0] += lo.x; acc[i][j][1] += lo.y;
+                        acc[i][j][2] += hi.x; acc[i][j][3] += hi.y;
+                    }
+            }
+        }
+        const int mb = sg.tm * BM + wm * 16 * MI + 2 * (AK ? sigma_row(g) : g);
+        const int nb = sg.tn * TBN + wn * 32 + 8 * t;
+        store_tile<MI>(prob, mb, nb, acc);
+    }
+
+    if (producer) {
+        // as above: no TMA write may land in shared memory after exit
+        const uint32_t from = issued > STAGES ? issued - STAGES : 0;
+        for (uint32_t L = from; L < issued; ++L) {
+            const uint32_t s = L % STAGES, ph = (L / STAGES) & 1u;
+            uint64_t t0 = global_timer_ns();
+            while (!mbar_try_wait(&full[s], ph)) {
+                if (global_timer_ns() - t0 > limit_ns) {
+                    atomicCAS(status, 0, CA3DMM_DEV_TIMEOUT_PRODUCE);
+                    break;
+                }
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_slot),
+                     "r"(TOTAL_COLS)
+                     : "memory");
+    }
+}
 
 typedef CUresult (*encode_tiled_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
                                     const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
@@ -593,6 +924,234 @@ extern "C" int ca3dmm_dgemm_launch_ranges_tn(const void *dev_plan, int nprob,
                                                      dev_status, limit, stream)
                        : dgemm_launch_one<false, 64>(grid, tm, dp, nprob, *ranges, total_tiles,
                                                       dev_status, limit, stream);
+    CA3DMM_CUDA_TRY(err);
+    ca3dmm_note_launch(1);
+    return CA3DMM_OK;
+}
+
+// ------------------------------------------------------------------ k segments, host side
+// The k segments of an m x n x k product, in tiles of 128 rows x 128 columns
+// taken in bands of 8 tile rows (the GEMM's raster order).  `grid` CTAs share
+// the tiles' 16-k blocks equally: after `whole` rounds of whole tiles (one tile
+// per CTA and round) the blocks of the remaining tiles are cut at multiples of
+// their number / grid.  The cuts depend on (m, n, k) alone, not on the tile
+// width, the raster or the operands' layout, and neither do the results.
+//
+// When (all in units of a 16-k block of one tile, 2.25 us of an SM): whole
+// tiles take ceil(T / 148) K.  Segments take T K / 148 and, for finishing cut
+// tiles, about 1.1 (writing a partial, the counter) and 0.4 per partial read
+// back.  At 1000^3 (T = 64, K = 63) that is 63 against 31: measured 148 us
+// against 70; at 2048^3 the sub-slabs of 512 k and their sum took 574 us, the
+// segments 523 (2.3 us per block of the 93 % busy tensor pipe, 3 us to start, 3
+// for the cut tiles).  Whole calls: 194 -> 124 and 629 -> 591 us; 1501 x 2003 x
+// 3001 with both operands transposed 747 -> 694; 200 x 150 x 300 77 -> 71.  A product of few blocks is not spread over all SMs: the
+// partials read back by the last CTA of a tile grow with the parts, so the
+// number of CTAs is at most sqrt(2.5 T T K).
+namespace {
+constexpr int SEG_SMS = 148, SEG_MAX_TILES = 16 * SEG_SMS, SEG_RASTER = 8;
+
+struct SegShape {
+    long long T, K;              // 128 x 128 tiles, 16-k blocks of a tile
+    int tiles_m, tiles_n, grid;
+    long long whole;             // rounds of whole tiles before the cut ones (-1: nothing is cut)
+};
+
+bool seg_shape(int m, int n, int k, SegShape &s)
+{
+    if (m <= 0 || n <= 0 || k <= 0) return false;
+    s.tiles_m = (m + 127) / 128;
+    s.tiles_n = (n + 127) / 128;
+    s.T = (long long) s.tiles_m * s.tiles_n;
+    s.K = ((long long) k + BK - 1) / BK;
+    if (s.T > SEG_MAX_TILES) return false;
+    const double dp = (double) ((s.T + SEG_SMS - 1) / SEG_SMS) * (double) s.K;
+    double g = std::sqrt(2.5 * (double) s.T * (double) s.T * (double) s.K);
+    if (g > SEG_SMS) g = SEG_SMS;
+    if (g > (double) (s.T * s.K)) g = (double) (s.T * s.K);
+    s.grid = g < 1.0 ? 1 : (int) g;
+    const double parts = s.T >= s.grid ? 2.0 : (double) s.grid / (double) s.T + 1.0;
+    const double seg = (double) s.T * (double) s.K / s.grid + 1.1 + 0.4 * parts;
+    if (seg < 0.98 * dp) {
+        s.whole = s.T / s.grid > 1 ? s.T / s.grid - 1 : 0;
+    } else {
+        s.whole = -1;
+        s.grid = s.T < SEG_SMS ? (int) s.T : SEG_SMS;
+    }
+    return true;
+}
+
+void seg_tile(const SegShape &s, long long tile, int &tm, int &tn)
+{
+    const long long per = (long long) SEG_RASTER * s.tiles_n, b = tile / per, r = tile % per;
+    const int first = (int) b * SEG_RASTER;
+    const int rows = s.tiles_m - first < SEG_RASTER ? s.tiles_m - first : SEG_RASTER;
+    tm = first + (int) (r % rows);
+    tn = (int) (r / rows);
+}
+}  // namespace
+
+extern "C" int ca3dmm_dgemm_segments_max(int m, int n, int k)
+{
+    SegShape s;
+    if (!seg_shape(m, n, k, s)) return 0;
+    // several rounds that cutting would not shorten: whole tiles in raster order
+    if (s.whole < 0 && s.T >= 4 * SEG_SMS) return 0;
+    return (int) (2 * (s.T + s.grid));
+}
+
+extern "C" size_t ca3dmm_dgemm_segments_ws_bytes(int m, int n, int k)
+{
+    SegShape s;
+    if (!seg_shape(m, n, k, s) || s.whole < 0) return 0;
+    // every cut adds one partial to the tile it falls into, whose first it also makes
+    return (size_t) 2 * (size_t) s.grid * BM * 128 * sizeof(double);
+}
+
+extern "C" int ca3dmm_dgemm_segments(int m, int n, int k, int tile_n, ca3dmm_dgemm_seg_t *segs,
+                                     int *order, int *cta_begin, int *nseg, int *grid,
+                                     int *ncounter)
+{
+    SegShape s;
+    *nseg = *grid = *ncounter = 0;
+    if (!seg_shape(m, n, k, s) || (tile_n != 128 && tile_n != 64)) return CA3DMM_EINVAL;
+    const int G = s.grid;
+    const long long dp = s.whole < 0 ? s.T : s.whole * G;       // whole tiles
+    const long long U = (s.T - dp) * s.K;                       // blocks of the others
+    // cut points in blocks; one within 1/16 of a share (or one block) of a tile's
+    // edge moves there, which saves a partial
+    const long long slack = U / G / 16 > 1 ? U / G / 16 : 1;
+    int ns = 0, nc = 0, slots = 0;
+    long long cut[SEG_SMS + 1];
+    for (int c = 0; c <= G; ++c) {
+        long long u = U > 0 ? U * c / G : 0;
+        if (c > 0 && c < G) {
+            const long long r = u % s.K;
+            if (r <= slack && r < s.K - r) u -= r;
+            else if (s.K - r <= slack) u += s.K - r;
+            if (u < cut[c - 1]) u = cut[c - 1];
+        }
+        cut[c] = u;
+    }
+    // segments in tile order, each with the CTA that runs it
+    int *who = static_cast<int *>(malloc(sizeof(int) * (size_t) (2 * (s.T + G) + 1)));
+    if (!who) return CA3DMM_ENOMEM;
+    int c = 0;                                                  // CTA holding block u
+    for (long long tile = 0; tile < s.T; ++tile) {
+        int tm, tn;
+        seg_tile(s, tile, tm, tn);
+        const int halves = tile_n == 128 ? 1 : (n - tn * 128 > 64 ? 2 : 1);
+        long long u0 = 0;
+        if (tile >= dp) {
+            u0 = (tile - dp) * s.K;
+            while (c + 1 < G && cut[c + 1] <= u0) ++c;
+        }
+        for (int h = 0; h < halves; ++h) {
+            int q = c, part = 0;
+            long long from = 0;
+            do {
+                ca3dmm_dgemm_seg_t &g = segs[ns];
+                long long to = s.K;
+                if (tile >= dp) {
+                    // skip CTAs left empty by moved cut points
+                    while (q + 1 < G && cut[q + 1] <= u0 + from) ++q;
+                    if (q + 1 < G && cut[q + 1] < u0 + s.K) to = cut[q + 1] - u0;
+                }
+                g.tm = tm;
+                g.tn = tile_n == 128 ? tn : 2 * tn + h;
+                g.kt0 = (int) from;
+                g.kt1 = (int) to;
+                g.part = part++;
+                g.nparts = 0;
+                g.slot0 = 0;
+                g.counter = 0;
+                who[ns++] = tile < dp ? (int) (tile % G) : q;
+                from = to;
+            } while (from < s.K);
+            for (int i = 0; i < part; ++i) {
+                ca3dmm_dgemm_seg_t &g = segs[ns - part + i];
+                g.nparts = part;
+                g.slot0 = part > 1 ? slots : 0;
+                g.counter = part > 1 ? nc : 0;
+            }
+            if (part > 1) { slots += part; ++nc; }
+        }
+    }
+    // per-CTA lists, in tile order
+    for (int b = 0; b <= G; ++b) cta_begin[b] = 0;
+    for (int i = 0; i < ns; ++i) ++cta_begin[who[i] + 1];
+    for (int b = 0; b < G; ++b) cta_begin[b + 1] += cta_begin[b];
+    int *at = static_cast<int *>(malloc(sizeof(int) * (size_t) (G + 1)));
+    if (!at) { free(who); return CA3DMM_ENOMEM; }
+    memcpy(at, cta_begin, sizeof(int) * (size_t) G);
+    for (int i = 0; i < ns; ++i) order[at[who[i]]++] = i;
+    free(at);
+    free(who);
+    *nseg = ns;
+    *grid = G;
+    *ncounter = nc;
+    return CA3DMM_OK;
+}
+
+namespace {
+template <bool AK, int TBN>
+cudaError_t seg_launch_one(int grid, const CUtensorMap *tm, const DProb &prob, const SegOrder &o,
+                           const ca3dmm_dgemm_seg_t *segs, double2 *partials, int *counters,
+                           int *status, unsigned long long limit, cudaStream_t stream)
+{
+    static std::atomic<unsigned long long> done{0};      // as dgemm_attr_once
+    int dev = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err != cudaSuccess) return err;
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+    if (!bit || !(done.load(std::memory_order_acquire) & bit)) {
+        err = cudaFuncSetAttribute(dgemm_dmma_segments<AK, TBN>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int) DTile<TBN>::SMEM_BYTES);
+        if (err != cudaSuccess) return err;
+        done.fetch_or(bit, std::memory_order_release);
+    }
+    dgemm_dmma_segments<AK, TBN><<<grid, THREADS, DTile<TBN>::SMEM_BYTES, stream>>>(
+        tm[0], tm[1], prob, o, segs, CA3DMM_DGEMM_CHUNK, partials, counters, status, limit);
+    return cudaGetLastError();
+}
+}  // namespace
+
+extern "C" int ca3dmm_dgemm_launch_segments(const void *host_plan, int nprob,
+                                            const ca3dmm_dgemm_seg_t *dev_segs,
+                                            const int *cta_begin, int lo, int hi, int grid,
+                                            int a_kmajor, void *partials, int *counters,
+                                            int *dev_status, double timeout_s, cudaStream_t stream,
+                                            int tile_n)
+{
+    if (tile_n != 128 && tile_n != 64) return CA3DMM_EINVAL;
+    if (hi <= lo) return CA3DMM_OK;
+    const CUtensorMap *tm = reinterpret_cast<const CUtensorMap *>(host_plan);
+    const DProb &prob = *reinterpret_cast<const DProb *>(tm + 2 * nprob);
+    SegOrder o;
+    memset(&o, 0, sizeof(o));
+    o.lists = cta_begin != nullptr;
+    o.lo = lo;
+    o.hi = hi;
+    if (cta_begin) {
+        if (grid < 1 || grid > CA3DMM_DGEMM_SEG_CTAS) return CA3DMM_EINVAL;
+        memcpy(o.begin, cta_begin, sizeof(int) * (size_t) (grid + 1));
+    } else {
+        grid = ca3dmm_device_sm_count();
+        if (grid > hi - lo) grid = hi - lo;
+    }
+    const unsigned long long limit = (unsigned long long) (timeout_s * 1e9);
+    double2 *ws = static_cast<double2 *>(partials);
+    cudaError_t err;
+    if (tile_n == 128)
+        err = a_kmajor ? seg_launch_one<true, 128>(grid, tm, prob, o, dev_segs, ws, counters,
+                                                    dev_status, limit, stream)
+                       : seg_launch_one<false, 128>(grid, tm, prob, o, dev_segs, ws, counters,
+                                                     dev_status, limit, stream);
+    else
+        err = a_kmajor ? seg_launch_one<true, 64>(grid, tm, prob, o, dev_segs, ws, counters,
+                                                   dev_status, limit, stream)
+                       : seg_launch_one<false, 64>(grid, tm, prob, o, dev_segs, ws, counters,
+                                                    dev_status, limit, stream);
     CA3DMM_CUDA_TRY(err);
     ca3dmm_note_launch(1);
     return CA3DMM_OK;
