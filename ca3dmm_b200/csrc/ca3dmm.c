@@ -34,10 +34,8 @@
 #define ALIGN_BYTES 256
 #define CANARY_BYTES 256
 #define CANARY_BYTE 0xA5
-/* the device status words, then the k segments' counters (cut tiles: at most one
- * per CTA boundary and half tile) */
-#define STATUS_WORDS_BYTES 64
-#define STATUS_BYTES (STATUS_WORDS_BYTES + 2 * CA3DMM_DGEMM_SEG_CTAS * (int) sizeof(int))
+/* the k segments' counters (cut tiles: at most one per CTA boundary and half tile) */
+#define COUNTER_BYTES (2 * CA3DMM_DGEMM_SEG_CTAS * (int) sizeof(int))
 
 typedef struct {
     int tk, tm, tn;        /* task ids */
@@ -66,7 +64,7 @@ typedef struct {
     group_t *groups;
     blk_t *A, *B;
     /* work buffer layout (byte offsets) */
-    size_t off_status, off_packA, off_packB, off_copy, off_tmapA, off_tmapB, off_gemm, off_ozplan;
+    size_t off_counters, off_packA, off_packB, off_copy, off_tmapA, off_tmapB, off_gemm, off_ozplan;
     size_t off_A, off_B, off_slab, off_cout, off_oz, total;
     size_t gemm_plan_bytes, oz_plan_bytes, oz_bytes;
     long long slab_ld;        /* leading dimension of each C slab */
@@ -74,7 +72,11 @@ typedef struct {
     /* pinned host staging for plan uploads */
     void *stage;
     size_t stage_bytes;
+    /* the status words of every launch: page-locked host memory that the kernels
+     * write where it lies (only when a bounded wait runs out or a guard band is
+     * overwritten), so an exec needs no clearing before and no copy after it */
     int *status_h;
+    int counters_clean;           /* the k segments' counters are zero (the last exec ended well) */
     /* cached exec arguments the device plan was built for */
     int plan_valid, c_ldA, c_ldB, c_ldC;
     const void *c_A, *c_B;
@@ -222,7 +224,7 @@ static void plan_layout(ca3dmm_engine_p e, plan_t *pl)
 {
     size_t off = 0;
     pl->ncanary = 0;
-    pl->off_status = off; off = align_up(off + STATUS_BYTES);
+    pl->off_counters = off; off = align_up(off + COUNTER_BYTES);
     pl->off_packA = off; off = align_up(off + sizeof(ca3dmm_pack_desc_t) * pl->nA);
     pl->off_packB = off; off = align_up(off + sizeof(ca3dmm_pack_desc_t) * pl->nB);
     pl->off_copy = off; off = align_up(off + sizeof(ca3dmm_pack_desc_t));
@@ -1243,7 +1245,7 @@ static int plan_upload(ca3dmm_engine_p e, const void *A, int ldA, const void *B,
         if (rc) return rc;
         e->crt_bits = pl->crt.p_min;
     }
-    memset(h + pl->off_status, 0, STATUS_BYTES);
+    memset(h + pl->off_counters, 0, COUNTER_BYTES);
     CA3DMM_CUDA_TRY(cudaMemcpyAsync(w, h, pl->stage_bytes, cudaMemcpyHostToDevice, st));
     for (int i = 0; i < pl->ncanary; i++)
         CA3DMM_CUDA_TRY(cudaMemsetAsync(w + pl->canary[i], CANARY_BYTE, CANARY_BYTES, st));
@@ -1265,7 +1267,7 @@ static int launch_pack_side(ca3dmm_engine_p e, int which, const void *src, cudaS
     if (which ? pl->packB_tma : pl->packA_tma)
         return ca3dmm_pack_tma_launch(w + (which ? pl->off_tmapB : pl->off_tmapA),
                                       (const ca3dmm_pack_desc_t *) (w + off_desc), nd, tiles,
-                                      (double *) w, (int *) (w + pl->off_status), 5.0, st);
+                                      (double *) w, pl->status_h, 5.0, st);
     return ca3dmm_pack_launch((const double *) src, (double *) w,
                               (const ca3dmm_pack_desc_t *) (w + off_desc), nd, tiles, st);
 }
@@ -1282,7 +1284,7 @@ static int launch_segments(ca3dmm_engine_p e, const ca3dmm_tile_ranges_t *rg, cu
     return ca3dmm_dgemm_launch_segments(
         (const char *) pl->stage + pl->off_gemm, pl->ngroup * pl->ksplit, sg,
         rg ? NULL : pl->seg_begin, lo, hi, pl->seg_grid, pl->a_kmajor, w + pl->off_slab,
-        (int *) (w + pl->off_status + STATUS_WORDS_BYTES), (int *) (w + pl->off_status), 5.0, st,
+        (int *) (w + pl->off_counters), pl->status_h, 5.0, st,
         pl->plain_tile_n);
 }
 
@@ -1301,6 +1303,16 @@ static int device_status_error(const plan_t *pl)
     }
     ERROR_PRINTF("Device status %d: a bounded wait ran out\n", code);
     return CA3DMM_ETIMEOUT;
+}
+
+/* The k segments' launches leave their counters zero; clear them when the last
+ * exec may not have ended (an asynchronous one, or one that failed), and always
+ * in an asynchronous exec, which may be captured and replayed. */
+static int counters_clear(plan_t *pl, char *w, int sync, cudaStream_t st)
+{
+    if (!pl->seg_plan || (sync && pl->counters_clean)) return CA3DMM_OK;
+    CA3DMM_CUDA_TRY(cudaMemsetAsync(w + pl->off_counters, 0, COUNTER_BYTES, st));
+    return CA3DMM_OK;
 }
 
 /* With CA3DMM_CANARY=1: compare every guard band with its fill pattern. */
@@ -1400,10 +1412,16 @@ static int exec_device(ca3dmm_engine_p e, const void *src_A, int ldA, const void
         pl->c_ldB != ldB || pl->c_dst != dst_C || pl->c_ldC != ldC) {
         rc = plan_upload(e, src_A, ldA, src_B, ldB, dst_C, ldC, st);
         if (rc) return rc;
-    } else if (cudaMemsetAsync(w + pl->off_status, 0, STATUS_BYTES, st) != cudaSuccess) {
-        return CA3DMM_ECUDA;
+    } else {
+        rc = counters_clear(pl, w, e->sync_exec, st);
+        if (rc) return rc;
     }
-    int timing = e->sync_exec && pl->events_ok;
+    pl->counters_clean = 0;
+    if (e->sync_exec) pl->status_h[0] = pl->status_h[1] = 0;
+    /* an event (about 5 us each) only where a phase begins or ends: plain FP64
+     * often neither packs nor sums, and a whole C needs no copy */
+    const int timing = e->sync_exec && pl->events_ok;
+    const int packs = e->gemm_mode != CA3DMM_GEMM_PLAIN || pl->pack_tiles_A > 0 || pl->pack_tiles_B > 0;
     if (timing) cudaEventRecord(pl->ev[0], st);
     const int crt = e->gemm_mode == CA3DMM_GEMM_CRT;
     /* NVTX ranges mark the phases of the reference's timers on the host
@@ -1420,8 +1438,8 @@ static int exec_device(ca3dmm_engine_p e, const void *src_A, int ldA, const void
     }
     nvtxRangePop();
     if (rc) return rc;
-    if (timing) cudaEventRecord(pl->ev[1], st);
-    int *status_d = (int *) (w + pl->off_status);
+    if (timing && packs) cudaEventRecord(pl->ev[1], st);
+    int *status_d = pl->status_h;
     nvtxRangePushA("ca3dmm: GEMM (2D Cannon)");
     int crt_bands = 0;
     if (crt) {
@@ -1468,8 +1486,9 @@ static int exec_device(ca3dmm_engine_p e, const void *src_A, int ldA, const void
         rc = ca3dmm_mirror_upper_launch(out, ldo, e->m, st);
     nvtxRangePop();
     if (rc) return rc;
-    if (timing) cudaEventRecord(pl->ev[3], st);
-    if (pl->has_dst && !whole) {
+    const int sums = crt || nred > 1 || pl->sym, copies = pl->has_dst && !whole;
+    if (timing && sums) cudaEventRecord(pl->ev[3], st);
+    if (copies) {
         nvtxRangePushA("ca3dmm: C to dst_C");
         rc = ca3dmm_pack_launch((const double *) (w + pl->off_cout), (double *) dst_C,
                                 (const ca3dmm_pack_desc_t *) (w + pl->off_copy), 1,
@@ -1477,21 +1496,20 @@ static int exec_device(ca3dmm_engine_p e, const void *src_A, int ldA, const void
         nvtxRangePop();
         if (rc) return rc;
     }
-    if (timing) cudaEventRecord(pl->ev[4], st);
+    if (timing && copies) cudaEventRecord(pl->ev[4], st);
     rc = launch_guard_check(e, pl, status_d, st);
     if (rc) return rc;
-    CA3DMM_CUDA_TRY(cudaMemcpyAsync(pl->status_h, status_d, 2 * sizeof(int), cudaMemcpyDeviceToHost,
-                                    st));
     if (e->sync_exec) {
         CA3DMM_CUDA_TRY(cudaStreamSynchronize(st));
         rc = device_status_error(pl);
         if (rc) return rc;
+        pl->counters_clean = 1;
         if (timing) {
             float t_pack = 0, t_gemm = 0, t_red = 0, t_copy = 0;
-            cudaEventElapsedTime(&t_pack, pl->ev[0], pl->ev[1]);
-            cudaEventElapsedTime(&t_gemm, pl->ev[1], pl->ev[2]);
-            cudaEventElapsedTime(&t_red, pl->ev[2], pl->ev[3]);
-            cudaEventElapsedTime(&t_copy, pl->ev[3], pl->ev[4]);
+            if (packs) cudaEventElapsedTime(&t_pack, pl->ev[0], pl->ev[1]);
+            cudaEventElapsedTime(&t_gemm, pl->ev[packs ? 1 : 0], pl->ev[2]);
+            if (sums) cudaEventElapsedTime(&t_red, pl->ev[2], pl->ev[3]);
+            if (copies) cudaEventElapsedTime(&t_copy, pl->ev[sums ? 3 : 2], pl->ev[4]);
             e->redist_ms += t_pack + t_copy;
             e->cannon_ms += t_gemm;
             e->reduce_ms += t_red;
@@ -1828,8 +1846,8 @@ static int hx_btb_slabs(ca3dmm_engine_p e, struct host_exec *x, const void *B_h,
         x->slab_built = 1;
     }
     char *w = (char *) e->workbuf_d;
-    int *status_d = (int *) (w + pl->off_status);
-    CA3DMM_CUDA_TRY(cudaMemsetAsync(status_d, 0, STATUS_BYTES, st));
+    int *status_d = pl->status_h;
+    status_d[0] = status_d[1] = 0;
     /* copies in: B slab by slab */
     for (int j = 0; j < kp; j++) {
         int k0, kz;
@@ -1892,8 +1910,6 @@ static int hx_btb_slabs(ca3dmm_engine_p e, struct host_exec *x, const void *B_h,
                                       (size_t) e->n, cudaMemcpyDeviceToHost, st));
     rc = launch_guard_check(e, pl, status_d, st);
     if (rc) return rc;
-    CA3DMM_CUDA_TRY(cudaMemcpyAsync(pl->status_h, status_d, 2 * sizeof(int), cudaMemcpyDeviceToHost,
-                                    st));
     CA3DMM_CUDA_TRY(cudaStreamSynchronize(st));
     return device_status_error(pl);
 }
@@ -1976,8 +1992,11 @@ static int exec_host(ca3dmm_engine_p e, const void *A_h, int ldA, const void *B_
         return CA3DMM_OK;
     }
     char *w = (char *) e->workbuf_d;
-    int *status_d = (int *) (w + pl->off_status);
-    CA3DMM_CUDA_TRY(cudaMemsetAsync(status_d, 0, STATUS_BYTES, st));
+    int *status_d = pl->status_h;
+    status_d[0] = status_d[1] = 0;
+    rc = counters_clear(pl, w, 1, st);
+    if (rc) return rc;
+    pl->counters_clean = 0;
     /* copies in: all of B, then the op(A) rows band by band */
     rc = hx_copy_in_B(e, x, B_h, ldB);
     if (rc) return rc;
@@ -2036,11 +2055,11 @@ static int exec_host(ca3dmm_engine_p e, const void *A_h, int ldA, const void *B_
     }
     rc = launch_guard_check(e, pl, status_d, st);
     if (rc) return rc;
-    CA3DMM_CUDA_TRY(cudaMemcpyAsync(pl->status_h, status_d, 2 * sizeof(int), cudaMemcpyDeviceToHost,
-                                    st));
     CA3DMM_CUDA_TRY(cudaStreamSynchronize(st));
     CA3DMM_CUDA_TRY(cudaStreamSynchronize(x->s_out));
-    return device_status_error(pl);
+    rc = device_status_error(pl);
+    pl->counters_clean = rc == CA3DMM_OK;
+    return rc;
 }
 
 int ca3dmm_engine_exec_host(ca3dmm_engine_p e, const void *A_h, int ldA, const void *B_h, int ldB,
