@@ -17,11 +17,11 @@
 //                         the next tile's MMAs).
 //                         The sums are exact (k 2^14 < 2^31); the epilogue reduces
 //                         each mod p_t into a byte plane of C's residues.
-//  4. crt_reconstruct_kernel<N, L> -- per C entry, C' from its N residues by the
-//                         Chinese remainder theorem: limb sums of the weights (in
-//                         constant memory), an FP64 quotient estimate, the low 128
-//                         bits exact; rounded once to double and scaled by
-//                         2^(E_i + F_j - 2P).
+//  4. crt_reconstruct_kernel<N> -- per C entry, C' from its N residues by the
+//                         Chinese remainder theorem: sums of three moduli at a time
+//                         in 32 bits, then limb sums of those, an FP64 quotient
+//                         estimate, the low 128 bits exact; rounded once to double
+//                         and scaled by 2^(E_i + F_j - 2P).
 //  5. crt_nonfinite_kernel -- rows / columns holding an Inf or a NaN were zero rows;
 //                         writes their entries' IEEE value.
 // Warp roles of the GEMM: warp 0 bulk-copy producer, warps 1-2 MMA issuers (two
@@ -50,6 +50,7 @@ constexpr int MAXMOD = CA3DMM_CRT_MAX_MODULI;
 constexpr int CBM = 128, CBN = 256, CKB = 128;   // tile rows, stored B tile rows, k bytes per stage
 constexpr int CA_BYTES = CBM * CKB;              // 16 KiB
 constexpr int CB_BYTES = CBN * CKB;              // 32 KiB
+constexpr int PL_BLOCK = 32 * CBM;               // C's residues: 32 columns of one tile row
 
 template <int TN>
 struct CrtTile {
@@ -67,56 +68,39 @@ constexpr int DEFAULT_BAND = 8;
 
 // ------------------------------------------------------------------ moduli
 // Pairwise coprime moduli <= 256, largest first (256 = 2^8 and odd numbers
-// with disjoint prime factors), and per modulus the constants of the GEMM
-// epilogue's reduction (2^16 mod p, floor(2^32 / p), a bias) and of the
-// residue pass (1/p in FP64).
+// with disjoint prime factors); per modulus the residue pass's 1/p in FP64, and
+// per modulus count and modulus the constants of the GEMM epilogue's reduction.
 constexpr int kModList[MAXMOD] = {256, 255, 253, 251, 247, 241, 239, 233, 229,
                                   227, 223, 217, 211, 199, 197, 193, 191, 181};
 static_assert(kModList[0] == 256, "the residue pass takes modulus 0 as the byte of the integer");
 
-struct ModConst {
-    int p, c16;          // p, 2^16 mod p
-    unsigned int mrec;   // floor(2^32 / p): floor(y mrec / 2^32) is floor(y / p) or one less (y < 2^28)
-    int bias;            // a multiple of p above 2^15 * 255 (keeps the epilogue's sums >= 0)
-    double inv;      // 1 / p rounded to double
-};
-
-constexpr ModConst make_mod(int p)
-{
-    return ModConst{p,
-                    (int) ((1LL << 16) % p),
-                    (unsigned int) ((1ULL << 32) / (unsigned long long) p),
-                    (int) (((8650752LL + p - 1) / p) * p),   // a multiple of p >= 2^23 + 2^18
-                    1.0 / (double) p};
-}
-
 struct ModTable {
-    ModConst m[MAXMOD];
+    struct { double inv; int p; } m[MAXMOD];
 };
 
 constexpr ModTable make_mod_table()
 {
     ModTable t{};
-    for (int i = 0; i < MAXMOD; ++i) t.m[i] = make_mod(kModList[i]);
+    for (int i = 0; i < MAXMOD; ++i) {
+        t.m[i].p = kModList[i];
+        t.m[i].inv = 1.0 / (double) kModList[i];
+    }
     return t;
 }
 
-// CRT weights, exact, for every modulus count N: M_N = prod_{t<N} p_t,
-// W_t = (M_N / p_t) ((M_N / p_t)^-1 mod p_t), so that sum_t u_t W_t = C' (mod M_N)
-// for residues u_t = C' mod p_t.  Little-endian 32-bit limbs.
-constexpr int LIMBS = 5;                        // M_18 < 2^141, W_t < M_N
+// Little-endian 32-bit limbs of the modulus products (M_18 < 2^141).
 struct Big {
     unsigned int w[6];
 };
 
-constexpr Big big_small(unsigned int v)
+__host__ __device__ constexpr Big big_small(unsigned int v)
 {
     Big b{};
     b.w[0] = v;
     return b;
 }
 
-constexpr Big big_mul(Big a, unsigned int m)
+__host__ __device__ constexpr Big big_mul(Big a, unsigned int m)
 {
     unsigned long long c = 0;
     for (int i = 0; i < 6; ++i) {
@@ -127,7 +111,7 @@ constexpr Big big_mul(Big a, unsigned int m)
     return a;
 }
 
-constexpr Big big_div(Big a, unsigned int d)
+__host__ __device__ constexpr Big big_div(Big a, unsigned int d)
 {
     unsigned long long r = 0;
     for (int i = 5; i >= 0; --i) {
@@ -152,40 +136,45 @@ constexpr unsigned int inv_mod(unsigned int a, unsigned int p)
     return 0;
 }
 
-struct CrtTable {
-    unsigned int W[MAXMOD + 1][MAXMOD][LIMBS];
-    unsigned int M[MAXMOD + 1][LIMBS + 1];
-    unsigned int H[MAXMOD + 1][LIMBS + 1];      // M / 2 (M is even: 256 is a modulus)
-    double Md[MAXMOD + 1], invM[MAXMOD + 1];
+__host__ __device__ constexpr Big mod_product(int n)
+{
+    Big M = big_small(1);
+    for (int t = 0; t < n; ++t) M = big_mul(M, (unsigned int) kModList[t]);
+    return M;
+}
+
+// The GEMM epilogue stores, for modulus t of N, u_t = v i_t mod p_t of the INT32
+// sum v, with i_t = (M_N / p_t)^-1 mod p_t: then sum_t u_t (M_N / p_t) = C' (mod
+// M_N), and the reconstruction needs no product with the inverses.
+struct EpiConst {
+    int p, inv, c16;     // p_t, i_t, i_t 2^16 mod p_t
+    unsigned int mrec;   // floor(2^32 / p): floor(y mrec / 2^32) is floor(y / p) or one less (y < 2^28)
+    int bias;            // a multiple of p above 2^15 * 255 (keeps the sums >= 0)
+};
+struct EpiTable {
+    EpiConst e[MAXMOD + 1][MAXMOD];
 };
 
-constexpr CrtTable make_crt_table()
+constexpr EpiTable make_epi_table()
 {
-    CrtTable T{};
+    EpiTable T{};
     for (int n = 2; n <= MAXMOD; ++n) {
-        Big M = big_small(1);
-        for (int t = 0; t < n; ++t) M = big_mul(M, (unsigned int) kModList[t]);
+        const Big M = mod_product(n);
         for (int t = 0; t < n; ++t) {
             const unsigned int p = (unsigned int) kModList[t];
-            Big Mt = big_div(M, p);
-            const Big W = big_mul(Mt, inv_mod(big_mod(Mt, p), p));
-            for (int q = 0; q < LIMBS; ++q) T.W[n][t][q] = W.w[q];
+            const unsigned int inv = inv_mod(big_mod(big_div(M, p), p), p);
+            T.e[n][t].p = (int) p;
+            T.e[n][t].inv = (int) inv;
+            T.e[n][t].c16 = (int) ((65536ull % p) * inv % p);
+            T.e[n][t].mrec = (unsigned int) ((1ULL << 32) / p);
+            T.e[n][t].bias = (int) (((8650752LL + p - 1) / p) * p);   // >= 2^23 + 2^18
         }
-        const Big H = big_div(M, 2);
-        double md = 0.0;
-        for (int q = 5; q >= 0; --q) md = md * 4294967296.0 + (double) M.w[q];
-        for (int q = 0; q <= LIMBS; ++q) {
-            T.M[n][q] = M.w[q];
-            T.H[n][q] = H.w[q];
-        }
-        T.Md[n] = md;
-        T.invM[n] = 1.0 / md;
     }
     return T;
 }
 
 __constant__ ModTable kMod = make_mod_table();
-__constant__ CrtTable kCrt = make_crt_table();
+__constant__ EpiTable kEpi = make_epi_table();
 
 double log2_modprod(int nmod)
 {
@@ -287,12 +276,12 @@ struct CrtGroup {
     int a_desc, b_desc, a_from_b;   // a_from_b: A tile tm is half tm % 2 of the B block's tile tm / 2
     int tiles_m, tiles_n, item_begin, band;
     int tile_n, pad_;               // GEMM tile columns (128 or 256; the same in every group)
-    long long rc_begin;             // first reconstruction item (4 rows x 1 column) of the group
+    long long rc_begin;             // first reconstruction item (128 rows x 2 columns) of the group
     int P, nkb;                     // integer width, 128-byte k blocks
     long long ea_off, eb_off;       // exponents of the A rows / B columns
     long long qa_off, qb_off;       // residue bytes of the operand blocks
     long long qa_tstride, qb_tstride;
-    long long pl_off, pl_ld, pl_bytes;   // residue planes of C: [t][tiles_n * 256][pl_ld]
+    long long pl_off;               // residues of C: [column / 32][tile row][t][column % 32][128 rows]
 };
 
 struct CrtHeader {
@@ -363,14 +352,15 @@ __device__ __forceinline__ uint64_t sdesc_sw128(uint32_t saddr)
     return d;
 }
 
-// int32 sum -> its residue mod p in [0, p): v = 2^16 h + l (h signed), so
-// y = h (2^16 mod p) + l + bias >= 0 is below 2^25 and congruent to v; the
-// quotient floor(y floor(2^32/p) / 2^32) is short by at most one.
-__device__ __forceinline__ unsigned int mod_i32(uint32_t vbits, const ModConst &mc)
+// int32 sum v -> v i mod p in [0, p): v = 2^16 h + l (h signed), so y = h (i 2^16
+// mod p) + l i + bias >= 0 is below 2^26 and congruent to v i; the quotient
+// floor(y floor(2^32/p) / 2^32) is short by at most one.
+__device__ __forceinline__ unsigned int mod_i32(uint32_t vbits, const EpiConst &mc)
 {
     const int v = (int) vbits;
     const int h = v >> 16;
-    const unsigned int y = (unsigned int) (h * mc.c16 + (int) (vbits & 0xffffu) + mc.bias);
+    const unsigned int y =
+        (unsigned int) (h * mc.c16 + ((int) (vbits & 0xffffu) * mc.inv + mc.bias));
     const unsigned int q = __umulhi(y, mc.mrec);
     const unsigned int r0 = y - q * (unsigned int) mc.p;
     const unsigned int r1 = r0 - (unsigned int) mc.p;
@@ -542,9 +532,16 @@ crt_gemm_kernel(const CrtGroup *__restrict__ groups, int ngroup, int nmod,
                                    CA3DMM_DEV_TIMEOUT_EPI, limit_ns))
                 break;
             tc_fence_after();
-            const ModConst mc = kMod.m[t];
-            const int row = tm * CBM + q * 32 + lane;
-            unsigned char *plane = work + G.pl_off + (long long) t * G.pl_bytes + row;
+            const EpiConst mc = kEpi.e[nmod][t];
+            // C's residues lie [column / 32][tile row][modulus][column % 32][128 rows]: a
+            // warp's 32 columns of an accumulator go to one 4 KB run of the block, and the
+            // reconstruction reads every modulus of a piece of a column, both at offsets
+            // known when they are compiled.  (One plane per modulus: the addresses took
+            // a fifth of the reconstruction's instructions.  All moduli of a column's 128
+            // rows together: the stores here lay up to 30 KB apart, 100 -> 105 us for the
+            // GEMMs of 2048^3.)
+            unsigned char *plane = work + G.pl_off + ((long long) tm * nmod + t) * PL_BLOCK + q * 32 + lane;
+            const long long pl_col = (long long) G.tiles_m * nmod * PL_BLOCK;   // 32 columns on
             // columns past tile_cols were not accumulated (still zero) and lie
             // past the group's n (never read): skipped
             const int ncols = tile_cols(G, tn, TN);
@@ -556,10 +553,10 @@ crt_gemm_kernel(const CrtGroup *__restrict__ groups, int ngroup, int nmod,
                 const uint32_t ta = tmem_base + ((uint32_t) (q * 32) << 16) + buf * TN + (uint32_t) c0;
                 tmem_ld32(ta, vv);
                 tmem_zero32(ta);
-                unsigned char *pc = plane + (long long) (tn * TN + c0) * G.pl_ld;
+                unsigned char *pc = plane + ((tn * TN + c0) >> 5) * pl_col;
 #pragma unroll
                 for (int j = 0; j < 32; ++j)
-                    pc[(long long) j * G.pl_ld] = (unsigned char) mod_i32(vv[j], mc);
+                    pc[j * CBM] = (unsigned char) mod_i32(vv[j], mc);
             }
             tmem_wait_st();
             tc_fence_before();
@@ -596,42 +593,201 @@ __device__ __forceinline__ double u128_to_double(unsigned long long hi, unsigned
     return __ull2double_rn(w);
 }
 
-// 32-bit limbs that the modulus product M_N needs (known at compile time)
-constexpr int crt_limbs(int n)
+// The moduli in groups of two or three consecutive ones, product M_g < 2^24, for
+// the reconstruction with N moduli: in group g, Y_g = sum_t u_t (M_g / p_t) <
+// 3 M_g takes 16-bit weights and 32 bits, and S = sum_t u_t (M / p_t) =
+// sum_g Y_g (M / M_g) has a third of the limb products of the sum over t.
+template <int N>
+struct Recon {
+    static constexpr int G = (N + 2) / 3;
+    int begin[G + 1];
+    unsigned int w01[G], w2[G];        // M_g / p_t of the group's moduli, two 16-bit halves
+    unsigned int limb[G][4];           // M / M_g
+    unsigned int NM[4];                // 2^128 - M mod 2^128
+    int limbs;                         // limbs of the largest M / M_g
+    int shift;                         // the estimate takes S 2^-shift (below 2^52, above M 2^-shift >= 2^45)
+    double inv;                        // 2^shift / M
+};
+
+template <int N>
+__host__ __device__ constexpr Recon<N> make_recon()
 {
-    const CrtTable T = make_crt_table();
-    int l = LIMBS + 1;
-    while (l > 1 && T.M[n][l - 1] == 0u) --l;
-    return l;
+    Recon<N> R{};
+    constexpr int G = Recon<N>::G;
+    const Big M = mod_product(N);
+    unsigned long long c = 1;
+    for (int q = 0; q < 4; ++q) {
+        c += (unsigned int) ~M.w[q];
+        R.NM[q] = (unsigned int) c;
+        c >>= 32;
+    }
+    int at = 0;
+    R.limbs = 2;
+    for (int g = 0; g < G; ++g) {
+        R.begin[g] = at;
+        const int size = N / G + (g < N % G ? 1 : 0);
+        unsigned int mg = 1, w[3] = {0, 0, 0};
+        for (int t = 0; t < size; ++t) mg *= (unsigned int) kModList[at + t];
+        for (int t = 0; t < size; ++t) w[t] = mg / (unsigned int) kModList[at + t];
+        R.w01[g] = w[0] | (w[1] << 16);
+        R.w2[g] = w[2];
+        const Big L = big_div(M, mg);
+        for (int q = 0; q < 4; ++q) {
+            R.limb[g][q] = L.w[q];
+            if (L.w[q] && q + 1 > R.limbs) R.limbs = q + 1;
+        }
+        at += size;
+    }
+    R.begin[G] = at;
+    double md = 0.0;
+    for (int q = 5; q >= 0; --q) md = md * 4294967296.0 + (double) M.w[q];
+    // S < 18 M < 2^5 M; M has `bits` bits
+    int bits = 0;
+    for (int q = 5; q >= 0 && !bits; --q)
+        for (int i = 31; i >= 0 && !bits; --i)
+            if (M.w[q] >> i & 1) bits = 32 * q + i + 1;
+    R.shift = bits + 5 - 52;
+    double unit = 1.0;
+    for (int i = 0; i < R.shift; ++i) unit *= 2.0;
+    R.inv = unit / md;
+    return R;
 }
 
-// C' from its residues: S = sum_t u_t W_t (column sums of 32-bit limb
-// products), q = rint(S / M) from an FP64 estimate of S (|C'| < M / 2, and the
-// estimate is off by far less than the gap to a half-integer), then
-// C' = S - q M taken modulo 2^128, which holds it exactly in two's complement
-// because |C'| <= k 2^(2P) <= 2^123.  Only the limbs below 2^128 of S and q M
-// are formed; all W_t and M fit in L = crt_limbs(N) limbs (a template
-// argument, computed on the host).
-// Work items are 4 rows x 1 column of C.  One group: the rows [r0, r1) of
-// group g0; several: every row of groups [g0, g1), numbered by the groups'
-// rc_begin prefix (found by a search over a shared copy), so that the grid
-// is spread by size over a batch of uneven groups.
-template <int N, int L>
-__global__ void __launch_bounds__(256)
+// C' from its residues: S = sum_g Y_g (M / M_g) in 64-bit sums of 32-bit limb
+// products (Y_g < 2^26, so no sum overflows), q = rint(S / M) from an FP64
+// estimate of S's top bits (|C'| < M / 2, and the estimate is off by less than
+// 2^-40, far less than the gap to a half-integer), then C' = S - q M taken
+// modulo 2^128, which holds it exactly in two's complement because |C'| <= k
+// 2^(2P) <= 2^123.  The weights are compile-time constants.
+// What bounds it is instruction issue (about 125 per entry, half of the issue slots
+// of the 24 warps its 80 registers allow), then the planes' loads: 8000 x 8000
+// entries of 15 moduli in 458 us (two bands), 1.47 GB at 3.2 TB/s, 4.2 M entries
+// in 31 us.  With one limb product per modulus and limb, the value rounded through
+// a 64-bit window, and each lane storing its own rows, it took 270 instructions,
+// 914 and 61 us; 64 registers (launch bounds of four blocks) are within 1 %.
+// A warp takes 128 rows x 2 columns of C at a time (a work item): a lane the four
+// rows of one word of each plane, whose values go through shared memory so that
+// the stores run along the column (a lane that stored its own rows wrote an
+// eighth of a sector at a time).  One group: the rows [r0, r1) of group g0;
+// several: every row of groups [g0, g1), numbered by the groups' rc_begin prefix
+// (found by a search over a shared copy), so that the grid is spread by size over
+// a batch of uneven groups.
+constexpr int RC_ROWS = 128, RC_COLS = 2, RC_STAGE = RC_ROWS + RC_ROWS / 4;   // padded: lanes 5 doubles apart
+constexpr int RC_WARPS = 8;
+
+__host__ __device__ inline long long recon_items_of(int rows, int cols)
+{
+    return rows > 0 && cols > 0 ? (long long) ((rows + RC_ROWS - 1) / RC_ROWS) *
+                                      ((cols + RC_COLS - 1) / RC_COLS)
+                                : 0;
+}
+
+template <int N>
+__device__ __forceinline__ void reconstruct4(const uint32_t (&u4)[N], double *__restrict__ out)
+{
+    constexpr Recon<N> R = make_recon<N>();
+    constexpr int G = Recon<N>::G, L = R.limbs;
+    static_assert(L >= 2 && L <= 4, "limb range");
+    // bytes of a group's planes -> per entry one word of its residues (the fourth
+    // byte meets no weight)
+    uint32_t w[G][4];
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+        const int t = R.begin[g];
+        const bool three = R.begin[g + 1] - t == 3;
+        const uint32_t lo = __byte_perm(u4[t], u4[t + 1], 0x5140);
+        const uint32_t hi = __byte_perm(u4[t], u4[t + 1], 0x7362);
+        const uint32_t third = three ? u4[t + 2] : 0u;
+        w[g][0] = __byte_perm(lo, third, 0x0410);
+        w[g][1] = __byte_perm(lo, third, 0x0532);
+        w[g][2] = __byte_perm(hi, third, 0x0610);
+        w[g][3] = __byte_perm(hi, third, 0x0732);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        unsigned long long a[L];
+#pragma unroll
+        for (int q = 0; q < L; ++q) a[q] = 0ull;
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            unsigned int Y = __dp2a_lo(R.w01[g], w[g][e], 0u);
+            if (R.begin[g + 1] - R.begin[g] == 3) Y = __dp2a_hi(R.w2[g], w[g][e], Y);
+#pragma unroll
+            for (int q = 0; q < L; ++q) a[q] += (unsigned long long) Y * R.limb[g][q];
+        }
+        // S 2^-shift, an integer below 2^52, from the sums above bit 32 (L - 2): as
+        // the mantissa of 2^52 + S 2^-shift
+        constexpr int cut = R.shift - 32 * (L - 2);
+        static_assert(cut >= 0 && cut < 64, "the estimate's bits");
+        const unsigned long long below = a[L - 2] + (L > 2 ? a[L > 2 ? L - 3 : 0] >> 32 : 0ull);
+        const unsigned long long above = a[L - 1] + (below >> 32);
+        const unsigned long long est =
+            cut >= 32 ? above >> (cut >= 32 ? cut - 32 : 0)
+                      : (above << (cut < 32 ? 32 - cut : 0)) | ((unsigned int) below >> (cut < 32 ? cut : 0));
+        const double top = __hiloint2double((int) ((unsigned int) (est >> 32) | 0x43300000u),
+                                            (int) (unsigned int) est) - 4503599627370496.0;
+        const unsigned int qe =
+            (unsigned int) __double2loint(fma(top, R.inv, 6755399441055744.0));
+        // S - q M = S + q (2^128 - M) modulo 2^128, word by word
+        unsigned int x[4];
+        unsigned long long carry = 0ull;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const unsigned long long v =
+                (unsigned long long) qe * R.NM[q] + (q < L ? a[q < L ? q : 0] : 0ull) + carry;
+            x[q] = (unsigned int) v;
+            carry = v >> 32;
+        }
+        const long long hi = (long long) (((unsigned long long) x[3] << 32) | x[2]);
+        double val;
+        if (x[3] + 0x80000u < 0x100000u && x[3] + 1u > 1u) {
+            // 2^96 <= |C'| < 2^115 (about): C' = hi 2^64 + lo, |hi| < 2^51; m = lo 2^-12
+            // with its last bit set when any bit below is (round to odd: that bit lies
+            // well below the result's last one, so one rounding of hi 2^52 + m rounds
+            // as the exact C' would).  hi - 1 and 2^52 + m are made from their bits and
+            // one subtraction, and (hi - 1) 2^52 + (2^52 + m) is one FMA.
+            const unsigned long long lo = ((unsigned long long) x[1] << 32) | x[0];
+            const unsigned int m0 = (unsigned int) (lo >> 12) | min(x[0] & 0xfffu, 1u);
+            const double h1 = __hiloint2double((int) (x[3] + 0x43380000u), (int) x[2]) -
+                              6755399441055745.0;
+            val = fma(h1, 4503599627370496.0,
+                      __hiloint2double((int) ((x[1] >> 12) | 0x43300000u), (int) m0)) * 4096.0;
+        } else {
+            unsigned long long lo = ((unsigned long long) x[1] << 32) | x[0];
+            unsigned long long mag = (unsigned long long) hi;
+            const bool neg = hi < 0;
+            if (neg) {
+                lo = ~lo + 1ull;
+                mag = ~mag + (lo == 0ull ? 1ull : 0ull);
+            }
+            int sh;
+            const double dv = u128_to_double(mag, lo, &sh);
+            val = scale2(dv, sh);
+            if (neg) val = -val;
+        }
+        out[e] = val;
+    }
+}
+
+template <int N>
+__global__ void __launch_bounds__(32 * RC_WARPS)
 crt_reconstruct_kernel(const CrtGroup *__restrict__ groups, int g0, int g1, int r0, int r1,
                        long long total, const unsigned char *__restrict__ work)
 {
-    static_assert(L >= 2 && L <= LIMBS, "modulus product outside the limb range");
-    __shared__ long long s_rb[GROUP_CACHE];
+    extern __shared__ long long s_rb[];              // several groups: their first items
+    __shared__ double stage_all[RC_WARPS][RC_STAGE];
     const int ng = g1 - g0;
     const bool cached = ng > 1 && ng <= GROUP_CACHE;
-    if (cached)
+    if (cached) {
         for (int i = threadIdx.x; i < ng; i += blockDim.x) s_rb[i] = groups[g0 + i].rc_begin;
-    __syncthreads();
+        __syncthreads();
+    }
     const int *ework = reinterpret_cast<const int *>(work);
     const long long base = ng > 1 ? groups[g0].rc_begin : 0;
-    for (long long it = blockIdx.x * (long long) blockDim.x + threadIdx.x; it < total;
-         it += (long long) gridDim.x * blockDim.x) {
+    const int lane = threadIdx.x & 31;
+    double *stage = stage_all[threadIdx.x >> 5];
+    for (long long it = blockIdx.x * (long long) RC_WARPS + (threadIdx.x >> 5); it < total;
+         it += (long long) gridDim.x * RC_WARPS) {
         int gi = 0;
         if (ng > 1) {
             const long long a = base + it;
@@ -645,69 +801,51 @@ crt_reconstruct_kernel(const CrtGroup *__restrict__ groups, int g0, int g1, int 
         const CrtGroup &G = groups[g0 + gi];
         const int rb = ng > 1 ? 0 : max(r0, 0), re = ng > 1 ? G.m : min(r1, G.m);
         if (re <= rb) continue;
-        const int nq = (re - rb + 3) >> 2;
+        const int nq = (re - rb + RC_ROWS - 1) / RC_ROWS;
         const long long local = ng > 1 ? base + it - G.rc_begin : it;
-        if (local >= (long long) nq * G.n) continue;
-        const int j = (int) (local / nq), i0 = rb + 4 * (int) (local % nq);
-        const int fb = ework[G.eb_off + j];
-        const int Fj = fb ? fb - EXP_BIAS : 0;
-        uint32_t u4[N];
+        if (local >= recon_items_of(re - rb, G.n)) continue;
+        const int jp = local >> 32 ? (int) (local / nq)
+                                   : (int) ((unsigned int) local / (unsigned int) nq);
+        const int i0 = rb + RC_ROWS * (int) (local - (long long) jp * nq), j0 = RC_COLS * jp;
+        const int ncol = min(RC_COLS, G.n - j0);
+        uint32_t u4[RC_COLS][N];
+        // columns j0, j0 + 1 (j0 even) are neighbours in one block of 32
+        const unsigned char *pl = work + G.pl_off +
+                                  ((long long) (j0 >> 5) * G.tiles_m + i0 / CBM) * (N * PL_BLOCK) +
+                                  (j0 & 31) * CBM + 4 * lane;
 #pragma unroll
         for (int t = 0; t < N; ++t)
-            u4[t] = __ldg(reinterpret_cast<const unsigned int *>(
-                work + G.pl_off + (long long) t * G.pl_bytes + (long long) j * G.pl_ld + i0));
+            u4[0][t] = __ldg(reinterpret_cast<const unsigned int *>(pl + t * PL_BLOCK));
+        if (ncol > 1) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int i = i0 + e;
-            if (i < re) {
-                unsigned long long a[L];
+            for (int t = 0; t < N; ++t)
+                u4[1][t] = __ldg(reinterpret_cast<const unsigned int *>(pl + CBM + t * PL_BLOCK));
+        }
+        const int rows = re - i0;
+        int Ei[4];
 #pragma unroll
-                for (int q = 0; q < L; ++q) a[q] = 0ull;
+        for (int i = 0; i < 4; ++i) {
+            const int eb = 32 * i + lane < rows ? ework[G.ea_off + i0 + 32 * i + lane] : 0;
+            Ei[i] = (eb ? eb - EXP_BIAS : 0) - 2 * G.P;
+        }
+        double *c = G.C + i0 + (long long) j0 * G.ldc;
+        const long long ldc = G.ldc;
+        const int *ebp = ework + G.eb_off + j0;
 #pragma unroll
-                for (int t = 0; t < N; ++t) {
-                    const unsigned int u = __byte_perm(u4[t], 0u, 0x4440u | (unsigned int) e);
+        for (int h = 0; h < RC_COLS; ++h) {
+            if (h >= ncol) break;
+            const int fb = ebp[h];
+            const int Fj = fb ? fb - EXP_BIAS : 0;
+            double v[4];
+            reconstruct4<N>(u4[h], v);
+            __syncwarp();                            // the previous column's values are read
 #pragma unroll
-                    for (int q = 0; q < L; ++q) a[q] += (unsigned long long) u * kCrt.W[N][t][q];
-                }
-                // quotient: S = sum_q a_q 2^(32 q) in FP64 (each a_q < 2^46 exact)
-                double sd = (double) a[L - 1];
+            for (int e = 0; e < 4; ++e) stage[5 * lane + e] = v[e];
+            __syncwarp();
 #pragma unroll
-                for (int q = L - 2; q >= 0; --q) sd = fma(sd, 4294967296.0, (double) a[q]);
-                const unsigned int qe = (unsigned int) __double2int_rn(sd * kCrt.invM[N]);
-                // low 128 bits of S and of q M, then C' = S - q M mod 2^128
-                unsigned int s4[4];
-                unsigned long long c = 0ull;
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const unsigned long long x = (q < L ? a[q] : 0ull) + c;
-                    s4[q] = (unsigned int) x;
-                    c = x >> 32;
-                }
-                unsigned int t4[4];
-                unsigned long long pc = 0ull;
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const unsigned long long pm = (unsigned long long) qe * kCrt.M[N][q] + pc;
-                    t4[q] = (unsigned int) pm;
-                    pc = pm >> 32;
-                }
-                const unsigned long long slo = ((unsigned long long) s4[1] << 32) | s4[0];
-                const unsigned long long shi = ((unsigned long long) s4[3] << 32) | s4[2];
-                const unsigned long long tlo = ((unsigned long long) t4[1] << 32) | t4[0];
-                const unsigned long long thi = ((unsigned long long) t4[3] << 32) | t4[2];
-                unsigned long long lo = slo - tlo;
-                unsigned long long hi = shi - thi - (slo < tlo ? 1ull : 0ull);
-                const bool neg = (long long) hi < 0;
-                if (neg) {
-                    lo = ~lo + 1ull;
-                    hi = ~hi + (lo == 0ull ? 1ull : 0ull);
-                }
-                int sh;
-                const double dv = u128_to_double(hi, lo, &sh);
-                const int eb = ework[G.ea_off + i];
-                const int Ei = eb ? eb - EXP_BIAS : 0;
-                const double val = scale2(dv, sh + Ei + Fj - 2 * G.P);
-                G.C[i + (long long) j * G.ldc] = neg ? -val : val;
+            for (int i = 0; i < 4; ++i) {
+                const int r = 32 * i + lane;
+                if (r < rows) c[r + h * ldc] = scale2(stage[r + (r >> 2)], Ei[i] + Fj);
             }
         }
     }
@@ -884,7 +1022,7 @@ extern "C" int ca3dmm_crt_plan_encode(ca3dmm_crt_plan_t *pl, int nmod, int nA,
         o.band = G[g].band > 0 ? G[g].band : DEFAULT_BAND;
         o.item_begin = items;
         o.rc_begin = recon;
-        recon += (long long) ((o.m + 3) / 4) * (o.n > 0 ? o.n : 0);
+        recon += recon_items_of(o.m, o.n);
         o.P = db.p_bits;
         o.nkb = o.k > 0 ? db.nkb : 0;
         o.ea_off = da.e_off;
@@ -893,10 +1031,8 @@ extern "C" int ca3dmm_crt_plan_encode(ca3dmm_crt_plan_t *pl, int nmod, int nA,
         o.qb_off = db.q_off;
         o.qa_tstride = da.t_stride;
         o.qb_tstride = db.t_stride;
-        o.pl_ld = round_up(o.m > 0 ? o.m : 1, CBM);
-        o.pl_bytes = (long long) crt_plane_bytes(o.m, o.n);
         o.pl_off = (long long) qoff;
-        qoff += align256((size_t) nmod * (size_t) o.pl_bytes);
+        qoff += align256((size_t) nmod * crt_plane_bytes(o.m, o.n));
         items += nmod * o.tiles_m * o.tiles_n;
         if (o.tiles_m > 0) {
             pmin = o.P < pmin ? o.P : pmin;
@@ -1151,16 +1287,21 @@ extern "C" int ca3dmm_crt_run_reconstruct_capped(const ca3dmm_crt_plan_t *pl, in
     long long total = pl->recon_items;
     if (g1 - g0 == 1 && pl->ngroup == 1) {
         const long long hi = r1 < pl->group_m ? r1 : pl->group_m, lo = r0 > 0 ? r0 : 0;
-        total = hi > lo ? ((hi - lo + 3) / 4) * pl->group_n : 0;
+        total = recon_items_of((int) (hi - lo), pl->group_n);
     }
     const CrtLayout L(pl->nA + pl->nB, pl->ngroup);
     const CrtGroup *groups =
         reinterpret_cast<const CrtGroup *>(static_cast<const unsigned char *>(pl->dev_plan) + L.gr);
     const unsigned char *w = static_cast<const unsigned char *>(pl->dev_work);
     if (total <= 0) return CA3DMM_OK;
-    long long blocks = (total + 255) / 256;
-    const long long cap = max_blocks > 0 ? max_blocks : (long long) ca3dmm_device_sm_count() * 8;
+    // beside a GEMM the blocks that fit with it; alone, blocks of one item per
+    // warp for one group (no last round of half the blocks), of several for a
+    // batch (each block copies the groups' first items)
+    long long blocks = (total + RC_WARPS - 1) / RC_WARPS;
+    const long long cap = max_blocks > 0 ? max_blocks
+                          : g1 - g0 > 1 ? (long long) ca3dmm_device_sm_count() * 64 : 1LL << 30;
     if (blocks > cap) blocks = cap;
+    const size_t smem = g1 - g0 > 1 && g1 - g0 <= GROUP_CACHE ? sizeof(long long) * (size_t) (g1 - g0) : 0;
     // the same shared-memory carveout as the GEMM, so that blocks of this
     // kernel can share an SM with a GEMM CTA running beside it (a kernel
     // attribute of each device: set once per instantiation, device and
@@ -1174,12 +1315,12 @@ extern "C" int ca3dmm_crt_run_reconstruct_capped(const ca3dmm_crt_plan_t *pl, in
 #define CA3DMM_CRT_CASE(N)                                                                          \
     case N:                                                                                         \
         if (!(__atomic_load_n(&carveout_set[N], __ATOMIC_ACQUIRE) & dbit)) {                        \
-            CA3DMM_CUDA_TRY(cudaFuncSetAttribute(crt_reconstruct_kernel<N, crt_limbs(N)>,          \
+            CA3DMM_CUDA_TRY(cudaFuncSetAttribute(crt_reconstruct_kernel<N>,          \
                                                  cudaFuncAttributePreferredSharedMemoryCarveout,  \
                                                  (int) cudaSharedmemCarveoutMaxShared));          \
             __atomic_fetch_or(&carveout_set[N], dbit, __ATOMIC_RELEASE);                            \
         }                                                                                           \
-        crt_reconstruct_kernel<N, crt_limbs(N)><<<(unsigned) blocks, 256, 0, stream>>>(            \
+        crt_reconstruct_kernel<N><<<(unsigned) blocks, 32 * RC_WARPS, smem, stream>>>(            \
             groups, g0, g1, r0, r1, total, w);                                                     \
         break;
         CA3DMM_CRT_CASE(8) CA3DMM_CRT_CASE(9) CA3DMM_CRT_CASE(10) CA3DMM_CRT_CASE(11)
