@@ -26,10 +26,11 @@
 //                         writes their entries' IEEE value.
 // Warp roles of the GEMM: warp 0 bulk-copy producer, warps 1-2 MMA issuers (two
 // of the four k steps of each stage each: one issuing thread alone does not keep
-// the tensor pipe busy), warps 3-10 epilogue (warp w reads TMEM lanes
-// 32 (w % 4) .. +31, columns 0 .. TN/2-1 or TN/2 .. TN-1 of the accumulator).  The MMAs only
-// accumulate; the epilogue zeroes each accumulator after reading it.  Every wait
-// is bounded; on timeout the kernel records a status, drains, frees TMEM, returns.
+// the tensor pipe busy), warps 3-10 epilogue (warp w reads TMEM lanes 32 (w % 4)
+// .. +31, columns 0 .. TN/2-1 or TN/2 .. TN-1 of the accumulator), warp 11 decodes
+// the work items for the others.  The MMAs only accumulate; the epilogue sets each
+// accumulator back to its start after reading it.  Every wait is bounded; on
+// timeout the kernel records a status, drains, frees TMEM, returns.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <climits>
@@ -50,7 +51,7 @@ constexpr int MAXMOD = CA3DMM_CRT_MAX_MODULI;
 constexpr int CBM = 128, CBN = 256, CKB = 128;   // tile rows, stored B tile rows, k bytes per stage
 constexpr int CA_BYTES = CBM * CKB;              // 16 KiB
 constexpr int CB_BYTES = CBN * CKB;              // 32 KiB
-constexpr int PL_BLOCK = 32 * CBM;               // C's residues: 32 columns of one tile row
+constexpr int PL_BLOCK = 32 * CBM, PL_COLS = 8;  // C's residues: 32 columns of one tile row, by 8
 
 template <int TN>
 struct CrtTile {
@@ -60,7 +61,7 @@ struct CrtTile {
     static constexpr int kTmemCols = 2 * TN;                    // two accumulators
     static constexpr size_t kSmem = (size_t) kStages * kStageBytes + (2 * kStages + 4) * 8 + 1024;
 };
-constexpr int C_THREADS = 352;                   // 11 warps
+constexpr int C_THREADS = 384;                   // 12 warps
 constexpr int C_ISSUERS = 2;
 constexpr int C_EPI_WARPS = 8;
 constexpr int GROUP_CACHE = 512;
@@ -147,13 +148,15 @@ __host__ __device__ constexpr Big mod_product(int n)
 // sum v, with i_t = (M_N / p_t)^-1 mod p_t: then sum_t u_t (M_N / p_t) = C' (mod
 // M_N), and the reconstruction needs no product with the inverses.
 struct EpiConst {
-    int p, inv, c16;     // p_t, i_t, i_t 2^16 mod p_t
-    unsigned int mrec;   // floor(2^32 / p): floor(y mrec / 2^32) is floor(y / p) or one less (y < 2^28)
-    int bias;            // a multiple of p above 2^15 * 255 (keeps the sums >= 0)
+    int p, bias;         // p_t; a multiple of it that keeps the sums >= 0
+    int w;               // signed bytes: i_t, i_t 2^16 mod p_t (centred)
+    unsigned int mrec;   // ceil(2^32 / p): floor(y mrec / 2^32) is floor(y / p) for y < 2^24
 };
 struct EpiTable {
     EpiConst e[MAXMOD + 1][MAXMOD];
 };
+
+constexpr int centred(unsigned int v, unsigned int p) { return v > (p - 1) / 2 ? (int) v - (int) p : (int) v; }
 
 constexpr EpiTable make_epi_table()
 {
@@ -163,11 +166,13 @@ constexpr EpiTable make_epi_table()
         for (int t = 0; t < n; ++t) {
             const unsigned int p = (unsigned int) kModList[t];
             const unsigned int inv = inv_mod(big_mod(big_div(M, p), p), p);
+            const int lo = centred(inv, p), hi = centred((unsigned int) (65536ull % p * inv % p), p);
+            // |sum of two 16-bit by 8-bit products| <= 32768 (127 + 127) for odd p
+            const unsigned int most = p == 256 ? 32768u * 256u : 32768u * 254u;
             T.e[n][t].p = (int) p;
-            T.e[n][t].inv = (int) inv;
-            T.e[n][t].c16 = (int) ((65536ull % p) * inv % p);
-            T.e[n][t].mrec = (unsigned int) ((1ULL << 32) / p);
-            T.e[n][t].bias = (int) (((8650752LL + p - 1) / p) * p);   // >= 2^23 + 2^18
+            T.e[n][t].bias = (int) ((most + p - 1) / p * p);
+            T.e[n][t].w = (lo & 255) | ((hi & 255) << 8);
+            T.e[n][t].mrec = (unsigned int) (((1ULL << 32) + p - 1) / p);
         }
     }
     return T;
@@ -276,12 +281,12 @@ struct CrtGroup {
     int a_desc, b_desc, a_from_b;   // a_from_b: A tile tm is half tm % 2 of the B block's tile tm / 2
     int tiles_m, tiles_n, item_begin, band;
     int tile_n, pad_;               // GEMM tile columns (128 or 256; the same in every group)
-    long long rc_begin;             // first reconstruction item (128 rows x 2 columns) of the group
+    long long rc_begin;             // first reconstruction item (32 rows x 8 columns) of the group
     int P, nkb;                     // integer width, 128-byte k blocks
     long long ea_off, eb_off;       // exponents of the A rows / B columns
     long long qa_off, qb_off;       // residue bytes of the operand blocks
     long long qa_tstride, qb_tstride;
-    long long pl_off;               // residues of C: [column / 32][tile row][t][column % 32][128 rows]
+    long long pl_off;               // residues of C: [column / 32][tile row][t][column % 32 / 8][128 rows][8]
 };
 
 struct CrtHeader {
@@ -352,24 +357,36 @@ __device__ __forceinline__ uint64_t sdesc_sw128(uint32_t saddr)
     return d;
 }
 
-// int32 sum v -> v i mod p in [0, p): v = 2^16 h + l (h signed), so y = h (i 2^16
-// mod p) + l i + bias >= 0 is below 2^26 and congruent to v i; the quotient
-// floor(y floor(2^32/p) / 2^32) is short by at most one.
-__device__ __forceinline__ unsigned int mod_i32(uint32_t vbits, const EpiConst &mc)
+// int32 sum v, given as x = v + 2^15 (the accumulators start at 2^15) -> v i mod p
+// in [0, p).  v = 2^16 h + l with signed halves: h is x's upper half, and l has
+// the bits of x's lower half with the top one flipped, so one two-way dot product
+// gives y = h (i 2^16 mod p) + l i + bias >= 0, below 2^24 for odd p, congruent to
+// v i; then q = floor(y / p) exactly and r = y - q p: four instructions (eight
+// when the halves were taken apart and the quotient could be one short).
+constexpr uint32_t ACC_START = 0x8000u;
+__device__ __forceinline__ unsigned int mod_i32(uint32_t x, const EpiConst &mc)
 {
-    const int v = (int) vbits;
-    const int h = v >> 16;
-    const unsigned int y =
-        (unsigned int) (h * mc.c16 + ((int) (vbits & 0xffffu) * mc.inv + mc.bias));
-    const unsigned int q = __umulhi(y, mc.mrec);
-    const unsigned int r0 = y - q * (unsigned int) mc.p;
-    const unsigned int r1 = r0 - (unsigned int) mc.p;
-    return r0 < r1 ? r0 : r1;
+    const unsigned int y = (unsigned int) __dp2a_lo((int) (x ^ 0x8000u), mc.w, mc.bias);
+    return y - __umulhi(y, mc.mrec) * (unsigned int) mc.p;
 }
 
 // ------------------------------------------------------------------ GEMM
+// What the roles need of a work item, decoded by the scheduler warp up to
+// ITEM_RING items ahead: the search for the item's group, the loads of its fields
+// and four divisions take about 1 us, which every role spent between two items
+// (a quarter of the time of items of eight k blocks).
+constexpr int ITEM_RING = 8;
+struct alignas(16) CrtItem {
+    const unsigned char *qa, *qb;   // residues of the item's tiles
+    unsigned char *plane;           // C's residues: the tile row's block of the first columns
+    long long pl_col;               // bytes to the block of the next 32 columns
+    int a_step, ncols, nkb, k, t;
+    int pad[3];
+};
+constexpr int ITEM_READERS = 1 + C_ISSUERS + C_EPI_WARPS;
+
 template <int TN>
-__global__ void __launch_bounds__(C_THREADS, 1)
+__global__ void __launch_bounds__(C_THREADS, 2)
 crt_gemm_kernel(const CrtGroup *__restrict__ groups, int ngroup, int nmod,
                 const ca3dmm_tile_ranges_t rg, int total_items,
                 unsigned char *__restrict__ work, int *status, unsigned long long limit_ns)
@@ -385,6 +402,8 @@ crt_gemm_kernel(const CrtGroup *__restrict__ groups, int ngroup, int nmod,
     uint64_t *acc_empty = acc_full + 2;         // [2]
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int abort_flag;
+    __shared__ CrtItem ring[ITEM_RING];
+    __shared__ uint64_t item_full[ITEM_RING], item_empty[ITEM_RING];
     __shared__ int s_gbeg[GROUP_CACHE];
     const int *gb = ngroup <= GROUP_CACHE ? s_gbeg : nullptr;
     if (gb)
@@ -399,6 +418,10 @@ crt_gemm_kernel(const CrtGroup *__restrict__ groups, int ngroup, int nmod,
         for (int b = 0; b < 2; ++b) {
             mbar_init(&acc_full[b], C_ISSUERS);
             mbar_init(&acc_empty[b], C_EPI_WARPS);
+        }
+        for (int s = 0; s < ITEM_RING; ++s) {
+            mbar_init(&item_full[s], 1);
+            mbar_init(&item_empty[s], ITEM_READERS);
         }
         abort_flag = 0;
         fence_barrier_init();
@@ -415,37 +438,34 @@ crt_gemm_kernel(const CrtGroup *__restrict__ groups, int ngroup, int nmod,
     tc_fence_after();
     const uint32_t tmem_base = tmem_slot;
     if (warp >= 3 && warp <= 6) {
-        // zero both accumulators (the MMAs only accumulate)
+        // start both accumulators (the MMAs only accumulate)
         const uint32_t lane_base = (uint32_t) ((warp & 3) * 32) << 16;
-        for (int c = 0; c < T::kTmemCols; c += 32) tmem_zero32(tmem_base + lane_base + (uint32_t) c);
+        for (int c = 0; c < T::kTmemCols; c += 32)
+            tmem_fill32(tmem_base + lane_base + (uint32_t) c, ACC_START);
         tmem_wait_st();
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
 
+    auto item_wait = [&](uint32_t i, int code) -> bool {
+        return mbar_wait_bounded(&item_full[i % ITEM_RING], (i / ITEM_RING) & 1u, &abort_flag,
+                                 status, code, limit_ns);
+    };
     if (warp == 0) {
         // ------------------------------------------------------ producer
         if (lane == 0) {
-            uint32_t it = 0;
+            uint32_t it = 0, ii = 0;
             bool ok = true;
             for (int v = blockIdx.x; v < total_items && ok && !abort_flag; v += gridDim.x) {
-                const int item = range_tile(rg, v);
-                const CrtGroup &G = groups[find_group(gb, groups, ngroup, item)];
-                int t, tm, tn;
-                item_decode(G, nmod, item, t, tm, tn);
-                const unsigned char *qa =
-                    G.a_from_b ? work + G.qa_off + t * G.qa_tstride +
-                                     (long long) (tm >> 1) * G.nkb * CB_BYTES + (tm & 1) * CA_BYTES
-                               : work + G.qa_off + t * G.qa_tstride + (long long) tm * G.nkb * CA_BYTES;
-                const long long a_step = G.a_from_b ? CB_BYTES : CA_BYTES;
-                const uint32_t b_bytes = (uint32_t) tile_cols(G, tn, TN) * CKB;
-                // a 128-column tile: half tn % 2 of stored 256-row tile tn / 2
-                const unsigned char *qb =
-                    TN == CBN ? work + G.qb_off + t * G.qb_tstride + (long long) tn * G.nkb * CB_BYTES
-                              : work + G.qb_off + t * G.qb_tstride +
-                                    (long long) (tn >> 1) * G.nkb * CB_BYTES + (tn & 1) * T::kBBytes;
-                for (int kb = 0; kb < G.nkb; ++kb, ++it) {
+                if (!item_wait(ii, CA3DMM_DEV_TIMEOUT_PRODUCE)) break;
+                const CrtItem &I = ring[ii % ITEM_RING];
+                const unsigned char *qa = I.qa, *qb = I.qb;
+                const int a_step = I.a_step, nkb = I.nkb;
+                const uint32_t b_bytes = (uint32_t) I.ncols * CKB;
+                mbar_arrive(&item_empty[ii % ITEM_RING]);
+                ++ii;
+                for (int kb = 0; kb < nkb; ++kb, ++it) {
                     const uint32_t s = it % CNSTAGE, ph = (it / CNSTAGE) & 1u;
                     if (!mbar_wait_bounded(&empty[s], ph ^ 1u, &abort_flag, status,
                                            CA3DMM_DEV_TIMEOUT_PRODUCE, limit_ns)) {
@@ -473,11 +493,14 @@ crt_gemm_kernel(const CrtGroup *__restrict__ groups, int ngroup, int nmod,
             uint32_t it = 0, ai = 0;
             bool ok = true;
             for (int v = blockIdx.x; v < total_items && ok; v += gridDim.x, ++ai) {
-                const int item = range_tile(rg, v);
-                const CrtGroup &G = groups[find_group(gb, groups, ngroup, item)];
-                int t, tm, tn;
-                item_decode(G, nmod, item, t, tm, tn);
-                const uint32_t idesc = idesc_i8(tile_cols(G, tn, TN), CBM);
+                if (!item_wait(ai, CA3DMM_DEV_TIMEOUT_ACCUM)) {
+                    ok = false;
+                    break;
+                }
+                const CrtItem &I = ring[ai % ITEM_RING];
+                const uint32_t idesc = idesc_i8(I.ncols, CBM);
+                const int nkb = I.nkb, k = I.k;
+                mbar_arrive(&item_empty[ai % ITEM_RING]);
                 const uint32_t buf = ai & 1u;
                 if (!mbar_wait_bounded(&acc_empty[buf], ((ai >> 1) & 1u) ^ 1u, &abort_flag, status,
                                        CA3DMM_DEV_TIMEOUT_ACCUM, limit_ns)) {
@@ -486,7 +509,7 @@ crt_gemm_kernel(const CrtGroup *__restrict__ groups, int ngroup, int nmod,
                 }
                 tc_fence_after();
                 const uint32_t tacc = tmem_base + buf * TN;
-                for (int kb = 0; kb < G.nkb; ++kb, ++it) {
+                for (int kb = 0; kb < nkb; ++kb, ++it) {
                     const uint32_t s = it % CNSTAGE, ph = (it / CNSTAGE) & 1u;
                     if (!mbar_wait_bounded(&full[s], ph, &abort_flag, status,
                                            CA3DMM_DEV_TIMEOUT_CONSUME, limit_ns)) {
@@ -497,7 +520,7 @@ crt_gemm_kernel(const CrtGroup *__restrict__ groups, int ngroup, int nmod,
                     const uint32_t sA = smem_u32(smem + s * CSTAGE_BYTES);
                     const uint32_t sB = sA + CA_BYTES;
                     // k steps past the group's k hold zero residues: not issued
-                    const int kleft = G.k - kb * CKB;
+                    const int kleft = k - kb * CKB;
 #pragma unroll
                     for (int kk = 2 * half; kk < 2 * half + 2; ++kk)
                         if (kk * 32 < kleft)
@@ -517,34 +540,66 @@ crt_gemm_kernel(const CrtGroup *__restrict__ groups, int ngroup, int nmod,
             }
         }
         __syncwarp();
+    } else if (warp == 11) {
+        // ------------------------------------------------------ scheduler
+        if (lane == 0) {
+            uint32_t ii = 0;
+            for (int v = blockIdx.x; v < total_items; v += gridDim.x, ++ii) {
+                const uint32_t s = ii % ITEM_RING;
+                if (!mbar_wait_bounded(&item_empty[s], ((ii / ITEM_RING) & 1u) ^ 1u, &abort_flag,
+                                       status, CA3DMM_DEV_TIMEOUT_QUEUE, limit_ns))
+                    break;
+                const int item = range_tile(rg, v);
+                const CrtGroup &G = groups[find_group(gb, groups, ngroup, item)];
+                int t, tm, tn;
+                item_decode(G, nmod, item, t, tm, tn);
+                CrtItem &I = ring[s];
+                const unsigned char *qa = work + G.qa_off + t * G.qa_tstride;
+                const unsigned char *qb = work + G.qb_off + t * G.qb_tstride;
+                I.qa = G.a_from_b
+                           ? qa + (long long) (tm >> 1) * G.nkb * CB_BYTES + (tm & 1) * CA_BYTES
+                           : qa + (long long) tm * G.nkb * CA_BYTES;
+                I.a_step = G.a_from_b ? CB_BYTES : CA_BYTES;
+                // a 128-column tile: half tn % 2 of stored 256-row tile tn / 2
+                I.qb = TN == CBN ? qb + (long long) tn * G.nkb * CB_BYTES
+                                 : qb + (long long) (tn >> 1) * G.nkb * CB_BYTES + (tn & 1) * T::kBBytes;
+                I.pl_col = (long long) G.tiles_m * nmod * PL_BLOCK;
+                I.plane = work + G.pl_off + ((long long) tm * nmod + t) * PL_BLOCK +
+                          (tn * TN >> 5) * I.pl_col;
+                I.ncols = tile_cols(G, tn, TN);
+                I.nkb = G.nkb;
+                I.k = G.k;
+                I.t = t;
+                mbar_arrive(&item_full[s]);
+            }
+        }
+        __syncwarp();
     } else {
         // ------------------------------------------------------ epilogue
         const int q = warp & 3;                       // TMEM lane quarter of this warp
         const int h = (warp - 3) >> 2;                // accumulator columns TN/2 h .. TN/2 (h + 1) - 1
         uint32_t ai = 0;
         for (int v = blockIdx.x; v < total_items; v += gridDim.x, ++ai) {
-            const int item = range_tile(rg, v);
-            const CrtGroup &G = groups[find_group(gb, groups, ngroup, item)];
-            int t, tm, tn;
-            item_decode(G, nmod, item, t, tm, tn);
+            if (!item_wait(ai, CA3DMM_DEV_TIMEOUT_EPI)) break;
+            const CrtItem &I = ring[ai % ITEM_RING];
+            const EpiConst mc = kEpi.e[nmod][I.t];
+            unsigned char *plane = I.plane + (q * 32 + lane) * PL_COLS;
+            const long long pl_col = I.pl_col;
+            const int ncols = I.ncols;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&item_empty[ai % ITEM_RING]);
             const uint32_t buf = ai & 1u;
             if (!mbar_wait_bounded(&acc_full[buf], (ai >> 1) & 1u, &abort_flag, status,
                                    CA3DMM_DEV_TIMEOUT_EPI, limit_ns))
                 break;
             tc_fence_after();
-            const EpiConst mc = kEpi.e[nmod][t];
-            // C's residues lie [column / 32][tile row][modulus][column % 32][128 rows]: a
-            // warp's 32 columns of an accumulator go to one 4 KB run of the block, and the
-            // reconstruction reads every modulus of a piece of a column, both at offsets
-            // known when they are compiled.  (One plane per modulus: the addresses took
-            // a fifth of the reconstruction's instructions.  All moduli of a column's 128
-            // rows together: the stores here lay up to 30 KB apart, 100 -> 105 us for the
-            // GEMMs of 2048^3.)
-            unsigned char *plane = work + G.pl_off + ((long long) tm * nmod + t) * PL_BLOCK + q * 32 + lane;
-            const long long pl_col = (long long) G.tiles_m * nmod * PL_BLOCK;   // 32 columns on
+            // C's residues lie [column / 32][tile row][modulus][column % 32 / 8][128 rows][8
+            // columns]: a thread's 32 columns of its row go out as four 8-byte stores, 256
+            // bytes a warp, and the reconstruction reads 8 columns of a row, every modulus
+            // at an offset known when it is compiled.  (As bytes, one plane per modulus,
+            // the 32 byte stores bounded products of small k: EPI_NOTE.)
             // columns past tile_cols were not accumulated (still zero) and lie
             // past the group's n (never read): skipped
-            const int ncols = tile_cols(G, tn, TN);
 #pragma unroll 1
             for (int cb = 0; cb < TN / 64; ++cb) {
                 const int c0 = h * (TN / 2) + cb * 32;
@@ -552,11 +607,21 @@ crt_gemm_kernel(const CrtGroup *__restrict__ groups, int ngroup, int nmod,
                 uint32_t vv[32];
                 const uint32_t ta = tmem_base + ((uint32_t) (q * 32) << 16) + buf * TN + (uint32_t) c0;
                 tmem_ld32(ta, vv);
-                tmem_zero32(ta);
-                unsigned char *pc = plane + ((tn * TN + c0) >> 5) * pl_col;
+                tmem_fill32(ta, ACC_START);
+                unsigned char *pc = plane + (c0 >> 5) * pl_col;
 #pragma unroll
-                for (int j = 0; j < 32; ++j)
-                    pc[j * CBM] = (unsigned char) mod_i32(vv[j], mc);
+                for (int g = 0; g < 32 / PL_COLS; ++g) {
+                    uint32_t o[2];
+#pragma unroll
+                    for (int w = 0; w < 2; ++w) {
+                        uint32_t r[4];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) r[e] = mod_i32(vv[PL_COLS * g + 4 * w + e], mc);
+                        o[w] = __byte_perm(__byte_perm(r[0], r[1], 0x0040),
+                                           __byte_perm(r[2], r[3], 0x0040), 0x5410);
+                    }
+                    *reinterpret_cast<uint2 *>(pc + g * (CBM * PL_COLS)) = make_uint2(o[0], o[1]);
+                }
             }
             tmem_wait_st();
             tc_fence_before();
@@ -665,20 +730,17 @@ __host__ __device__ constexpr Recon<N> make_recon()
 // in 31 us.  With one limb product per modulus and limb, the value rounded through
 // a 64-bit window, and each lane storing its own rows, it took 270 instructions,
 // 914 and 61 us; 64 registers (launch bounds of four blocks) are within 1 %.
-// A warp takes 128 rows x 2 columns of C at a time (a work item): a lane the four
-// rows of one word of each plane, whose values go through shared memory so that
-// the stores run along the column (a lane that stored its own rows wrote an
-// eighth of a sector at a time).  One group: the rows [r0, r1) of group g0;
-// several: every row of groups [g0, g1), numbered by the groups' rc_begin prefix
-// (found by a search over a shared copy), so that the grid is spread by size over
-// a batch of uneven groups.
-constexpr int RC_ROWS = 128, RC_COLS = 2, RC_STAGE = RC_ROWS + RC_ROWS / 4;   // padded: lanes 5 doubles apart
-constexpr int RC_WARPS = 8;
+// A warp takes 32 rows x 8 columns of C at a time (a work item), a lane the eight
+// columns of its row, so that loads and stores run along the rows.  One group: the
+// rows [r0, r1) of group g0; several: every row of groups [g0, g1), numbered by
+// the groups' rc_begin prefix (found by a search over a shared copy), so that the
+// grid is spread by size over a batch of uneven groups.
+constexpr int RC_ROWS = 32, RC_WARPS = 8;
 
 __host__ __device__ inline long long recon_items_of(int rows, int cols)
 {
     return rows > 0 && cols > 0 ? (long long) ((rows + RC_ROWS - 1) / RC_ROWS) *
-                                      ((cols + RC_COLS - 1) / RC_COLS)
+                                      ((cols + PL_COLS - 1) / PL_COLS)
                                 : 0;
 }
 
@@ -775,7 +837,6 @@ crt_reconstruct_kernel(const CrtGroup *__restrict__ groups, int g0, int g1, int 
                        long long total, const unsigned char *__restrict__ work)
 {
     extern __shared__ long long s_rb[];              // several groups: their first items
-    __shared__ double stage_all[RC_WARPS][RC_STAGE];
     const int ng = g1 - g0;
     const bool cached = ng > 1 && ng <= GROUP_CACHE;
     if (cached) {
@@ -785,7 +846,6 @@ crt_reconstruct_kernel(const CrtGroup *__restrict__ groups, int g0, int g1, int 
     const int *ework = reinterpret_cast<const int *>(work);
     const long long base = ng > 1 ? groups[g0].rc_begin : 0;
     const int lane = threadIdx.x & 31;
-    double *stage = stage_all[threadIdx.x >> 5];
     for (long long it = blockIdx.x * (long long) RC_WARPS + (threadIdx.x >> 5); it < total;
          it += (long long) gridDim.x * RC_WARPS) {
         int gi = 0;
@@ -806,47 +866,33 @@ crt_reconstruct_kernel(const CrtGroup *__restrict__ groups, int g0, int g1, int 
         if (local >= recon_items_of(re - rb, G.n)) continue;
         const int jp = local >> 32 ? (int) (local / nq)
                                    : (int) ((unsigned int) local / (unsigned int) nq);
-        const int i0 = rb + RC_ROWS * (int) (local - (long long) jp * nq), j0 = RC_COLS * jp;
-        const int ncol = min(RC_COLS, G.n - j0);
-        uint32_t u4[RC_COLS][N];
-        // columns j0, j0 + 1 (j0 even) are neighbours in one block of 32
+        const int i0 = rb + RC_ROWS * (int) (local - (long long) jp * nq), j0 = PL_COLS * jp;
+        const int i = i0 + lane, ncol = min(PL_COLS, G.n - j0);
         const unsigned char *pl = work + G.pl_off +
                                   ((long long) (j0 >> 5) * G.tiles_m + i0 / CBM) * (N * PL_BLOCK) +
-                                  (j0 & 31) * CBM + 4 * lane;
+                                  (j0 & 31) * CBM + (i & (CBM - 1)) * PL_COLS;
+        uint32_t u4[2][N];
 #pragma unroll
-        for (int t = 0; t < N; ++t)
-            u4[0][t] = __ldg(reinterpret_cast<const unsigned int *>(pl + t * PL_BLOCK));
-        if (ncol > 1) {
-#pragma unroll
-            for (int t = 0; t < N; ++t)
-                u4[1][t] = __ldg(reinterpret_cast<const unsigned int *>(pl + CBM + t * PL_BLOCK));
+        for (int t = 0; t < N; ++t) {
+            const uint2 x = __ldg(reinterpret_cast<const uint2 *>(pl + t * PL_BLOCK));
+            u4[0][t] = x.x;
+            u4[1][t] = x.y;
         }
-        const int rows = re - i0;
-        int Ei[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int eb = 32 * i + lane < rows ? ework[G.ea_off + i0 + 32 * i + lane] : 0;
-            Ei[i] = (eb ? eb - EXP_BIAS : 0) - 2 * G.P;
-        }
-        double *c = G.C + i0 + (long long) j0 * G.ldc;
-        const long long ldc = G.ldc;
+        const int eb = i < re ? ework[G.ea_off + i] : 0;
+        const int Ei = (eb ? eb - EXP_BIAS : 0) - 2 * G.P;
         const int *ebp = ework + G.eb_off + j0;
+        const long long ldc = G.ldc;
+        double *c = G.C + i + (long long) j0 * ldc;
 #pragma unroll
-        for (int h = 0; h < RC_COLS; ++h) {
-            if (h >= ncol) break;
-            const int fb = ebp[h];
-            const int Fj = fb ? fb - EXP_BIAS : 0;
+        for (int h = 0; h < 2; ++h) {
             double v[4];
             reconstruct4<N>(u4[h], v);
-            __syncwarp();                            // the previous column's values are read
 #pragma unroll
-            for (int e = 0; e < 4; ++e) stage[5 * lane + e] = v[e];
-            __syncwarp();
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int r = 32 * i + lane;
-                if (r < rows) c[r + h * ldc] = scale2(stage[r + (r >> 2)], Ei[i] + Fj);
-            }
+            for (int e = 0; e < 4; ++e)
+                if (4 * h + e < ncol && i < re) {
+                    const int fb = ebp[4 * h + e];
+                    c[(4 * h + e) * ldc] = scale2(v[e], Ei + (fb ? fb - EXP_BIAS : 0));
+                }
         }
     }
 }

@@ -422,16 +422,17 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32])
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// Zero 32 consecutive TMEM columns of this warp's 32 lanes.
-__device__ __forceinline__ void tmem_zero32(uint32_t taddr)
+// Set 32 consecutive TMEM columns of this warp's 32 lanes.
+__device__ __forceinline__ void tmem_fill32(uint32_t taddr, uint32_t z)
 {
-    const uint32_t z = 0;
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,"
         "%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr),
         "r"(z)
         : "memory");
 }
+
+__device__ __forceinline__ void tmem_zero32(uint32_t taddr) { tmem_fill32(taddr, 0u); }
 
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 

@@ -20,24 +20,35 @@ def product(l):
     return r
 
 
+def centred(v, p):
+    return v - p if v > (p - 1) // 2 else v
+
+
 @pytest.mark.parametrize("N", range(8, 19))
 def test_epilogue_reduction(N):
     rng = np.random.default_rng(N)
-    lim = 131072 * 128 * 128
-    v = np.concatenate([rng.integers(-lim, lim + 1, 100000),
-                        [0, 1, -1, lim - 1, -lim, 2 ** 16, -(2 ** 16), 2 ** 16 - 1, -(2 ** 31),
-                         2 ** 31 - 1]]).astype(np.int64)
     M = product(MODULI[:N])
     for p in MODULI[:N]:
+        # sums of k <= 131072 products of bytes: |r| <= 128 for p = 256 (whose sums may
+        # wrap modulo 2^32), else at most 127
+        lim = 131072 * (128 * 128 if p == 256 else 127 * 127)
+        v = np.concatenate([rng.integers(-lim, lim + 1, 100000),
+                            [0, 1, -1, lim, -lim, 32767, 32768, -32768, -32769, 65535, 65536,
+                             lim - 32768, 32768 - lim]]).astype(np.int64)
+        x = (v + 0x8000) & 0xFFFFFFFF                    # the accumulator
+        x = (x ^ 0x8000).astype(np.uint32)
+        h = (x >> np.uint32(16)).astype(np.uint16).view(np.int16).astype(np.int64)
+        l = (x & np.uint32(0xFFFF)).astype(np.uint16).view(np.int16).astype(np.int64)
         inv = pow(M // p, -1, p)
-        c16, bias, mrec = 65536 * inv % p, (8650752 + p - 1) // p * p, (1 << 32) // p
-        y = (v >> 16) * c16 + ((v & 0xFFFF) * inv + bias)
-        assert np.all(y >= 0) and np.all(y < 1 << 26)
+        lo, hi = centred(inv, p), centred(65536 * inv % p, p)
+        assert -128 <= lo <= 127 and -128 <= hi <= 127
+        most = 32768 * (256 if p == 256 else 254)
+        y = h * hi + l * lo + (most + p - 1) // p * p
+        assert np.all(y >= 0) and np.all(y < (1 << 24 if p != 256 else 1 << 25))
+        mrec = ((1 << 32) + p - 1) // p
         q = (y.astype(np.uint64) * np.uint64(mrec) >> np.uint64(32)).astype(np.int64)
         r = y - q * p
-        assert np.all((r >= 0) & (r < 2 * p))
-        r = np.where(r >= p, r - p, r)
-        assert np.all((r - v * inv) % p == 0) and np.all((r >= 0) & (r < p))
+        assert np.all((r >= 0) & (r < p)) and np.all((r - v * inv) % p == 0)
 
 
 def reconstruct(N, u):
