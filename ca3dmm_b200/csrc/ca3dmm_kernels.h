@@ -141,6 +141,17 @@ int ca3dmm_pack_launch(const double *src_base, double *dst_base,
                        const ca3dmm_pack_desc_t *dev_descs, int ndesc, int total_tiles,
                        cudaStream_t stream);
 
+/* Copies of up to CA3DMM_MAX_RUN_PIECES blocks in one launch, stream-ordered, the
+ * blocks passed as kernel arguments: `runs` runs of `len` contiguous elements,
+ * lds / ldd elements apart.  CA3DMM_EINVAL above that number of blocks. */
+#define CA3DMM_MAX_RUN_PIECES 512
+typedef struct {
+    const double *src;
+    double *dst;
+    int lds, ldd, len, runs;
+} ca3dmm_run_piece_t;
+int ca3dmm_copy_runs_launch(const ca3dmm_run_piece_t *pieces, int n, cudaStream_t stream);
+
 /* One column-major block copy dst[r + c*ldd] = src[r + c*lds] (rows x cols),
  * stream-ordered, the geometry passed as kernel arguments. */
 int ca3dmm_copy_block_launch(const double *src, long long lds, double *dst, long long ldd,

@@ -249,6 +249,96 @@ copy_block_kernel(const double *__restrict__ src, long long lds, double *__restr
     }
 }
 
+// Copies of many blocks with unrelated addresses and leading dimensions, the
+// blocks given in the launch's parameters.  HBM bound.  The contiguous runs of a
+// block are a few KB and start anywhere (layouts split a matrix into strips of any
+// width), so a warp copies whole runs, two at a time with all their loads in
+// flight, four per item, up to RUN_E elements of them; its stores cover whole
+// lines.  Items go through the blocks in turn, four runs of each, so that the
+// blocks that share a destination row fill it at about the same time.
+// 8000 x 8000 from 24 column strips to 4 x 6 blocks (116 pieces, 1.02 GB): 178 us,
+// 5.75 TB/s (one piece after the other 199-214; with default loads and stores in
+// place of the streaming ones, lines aligned, 373; 64 x 64 tiles from descriptors
+// in memory 206).  The call: 242 -> 206 us, with the upload of the descriptors and
+// the wait before it gone.
+constexpr int RUN_E = 512, RUN_GROUP = 4;
+__host__ __device__ inline int run_chunks(int len) { return (len + 15 + RUN_E - 1) / RUN_E; }
+
+template <int CAP>
+struct RunPieces {
+    ca3dmm_run_piece_t p[CAP];
+};
+
+template <int CAP>
+__global__ void __launch_bounds__(256)
+copy_runs_kernel(const __grid_constant__ RunPieces<CAP> P, int npiece, int nch, int total_items)
+{
+    const int lane = threadIdx.x & 31;
+    for (int item = blockIdx.x * 8 + (threadIdx.x >> 5); item < total_items; item += gridDim.x * 8) {
+        const int ic = item / nch, g = ic / npiece;
+        const ca3dmm_run_piece_t &d = P.p[ic - g * npiece];
+        const int c0 = (item - ic * nch) * RUN_E + lane;
+        const int r1 = min(d.runs, (g + 1) * RUN_GROUP);
+        if (g * RUN_GROUP >= d.runs || c0 - lane >= d.len + 15) continue;
+        for (int r = g * RUN_GROUP; r < r1; r += 2) {
+            // each run's elements counted from the 128-byte line its destination starts
+            // in, so that a warp's store covers whole lines
+            const double *s0 = d.src + (long long) r * d.lds;
+            double *t0 = d.dst + (long long) r * d.ldd, *t1 = t0 + d.ldd;
+            const int e0 = c0 - (int) ((reinterpret_cast<uintptr_t>(t0) >> 3) & 15);
+            const int e1 = c0 - (int) ((reinterpret_cast<uintptr_t>(t1) >> 3) & 15);
+            const unsigned int len = (unsigned int) d.len, len1 = r + 1 < r1 ? len : 0u;
+            s0 += e0;
+            const double *s1 = d.src + (long long) (r + 1) * d.lds + e1;
+            t0 += e0;
+            t1 += e1;
+            double v0[RUN_E / 32], v1[RUN_E / 32];
+#pragma unroll
+            for (int u = 0; u < RUN_E / 32; ++u) {
+                if ((unsigned int) (e0 + 32 * u) < len) v0[u] = __ldcs(s0 + 32 * u);
+                if ((unsigned int) (e1 + 32 * u) < len1) v1[u] = __ldcs(s1 + 32 * u);
+            }
+#pragma unroll
+            for (int u = 0; u < RUN_E / 32; ++u) {
+                if ((unsigned int) (e0 + 32 * u) < len) __stcs(t0 + 32 * u, v0[u]);
+                if ((unsigned int) (e1 + 32 * u) < len1) __stcs(t1 + 32 * u, v1[u]);
+            }
+        }
+    }
+}
+
+template <int CAP>
+static cudaError_t copy_runs_launch(const ca3dmm_run_piece_t *pieces, int n, cudaStream_t stream)
+{
+    RunPieces<CAP> P;
+    memset(&P, 0, sizeof(P));
+    long long groups = 0, nch = 0;
+    for (int i = 0; i < n; ++i) {
+        P.p[i] = pieces[i];
+        const long long g = pieces[i].len > 0 ? (pieces[i].runs + RUN_GROUP - 1) / RUN_GROUP : 0;
+        if (g > groups) groups = g;
+        if (run_chunks(pieces[i].len) > nch) nch = run_chunks(pieces[i].len);
+    }
+    const long long items = groups * n * nch;
+    if (items == 0) return cudaSuccess;
+    if (items > 0x7fffffffLL - 1000000) return cudaErrorInvalidValue;
+    const long long blocks = (items + 7) / 8, cap = (long long) ca3dmm_device_sm_count() * 64;
+    copy_runs_kernel<CAP><<<(unsigned) (blocks < cap ? blocks : cap), 256, 0, stream>>>(
+        P, n, (int) nch, (int) items);
+    ca3dmm_note_launch(1);
+    return cudaGetLastError();
+}
+
+extern "C" int ca3dmm_copy_runs_launch(const ca3dmm_run_piece_t *pieces, int n, cudaStream_t stream)
+{
+    if (n < 0 || n > CA3DMM_MAX_RUN_PIECES) return CA3DMM_EINVAL;
+    if (n == 0) return CA3DMM_OK;
+    // two parameter sizes: small launches carry less
+    CA3DMM_CUDA_TRY(n <= 64 ? copy_runs_launch<64>(pieces, n, stream)
+                            : copy_runs_launch<CA3DMM_MAX_RUN_PIECES>(pieces, n, stream));
+    return CA3DMM_OK;
+}
+
 extern "C" int ca3dmm_copy_block_launch(const double *src, long long lds, double *dst,
                                         long long ldd, int rows, int cols, cudaStream_t stream)
 {

@@ -139,6 +139,7 @@ struct mat_redist_layouts {
     int nsrc, nreq, npiece;
     int *src_rects, *req_rects;
     piece_t *pieces;
+    int by_value;                 /* few enough pieces to travel with the launch */
     ca3dmm_pack_desc_t *desc_h;   /* pinned staging of the descriptors */
     ca3dmm_pack_desc_t *desc_d;
 };
@@ -177,7 +178,14 @@ int mat_redist_layouts_init(int nsrc, const int *src_rects, int nreq, const int 
             p->src = i; p->dst = j;
             p->srow = r0; p->scol = c0; p->nrow = r1 - r0; p->ncol = c1 - c0;
         }
-    if (L->npiece > 0) {
+    double runs = 0, len = 0;     /* bound the launch's work items */
+    for (int k = 0; k < L->npiece; k++) {
+        if (L->pieces[k].nrow > runs) runs = L->pieces[k].nrow;
+        if (L->pieces[k].ncol > len) len = L->pieces[k].ncol;
+    }
+    L->by_value = L->npiece <= CA3DMM_MAX_RUN_PIECES &&
+                  (runs / 4 + 1) * (len / 512 + 2) * L->npiece < 1e9;
+    if (L->npiece > 0 && !L->by_value) {
         const size_t bytes = sizeof(ca3dmm_pack_desc_t) * (size_t) L->npiece;
         if (cudaMallocHost((void **) &L->desc_h, bytes) != cudaSuccess) L->desc_h = NULL;
         if (cudaMalloc((void **) &L->desc_d, bytes) != cudaSuccess) L->desc_d = NULL;
@@ -203,6 +211,26 @@ int mat_redist_layouts_exec(mat_redist_layouts_p L, const void *const *src_blks,
         if (dst_lds[j] < L->req_rects[4 * j + 3] || ((uintptr_t) dst_blks[j] & 7)) return CA3DMM_EINVAL;
     if (L->npiece == 0) return CA3DMM_OK;
     cudaStream_t st = (cudaStream_t) stream;
+    if (L->by_value) {
+        /* the pieces travel with the launch: no staging to wait for, no upload */
+        ca3dmm_run_piece_t rp[CA3DMM_MAX_RUN_PIECES];
+        for (int k = 0; k < L->npiece; k++) {
+            const piece_t *p = &L->pieces[k];
+            const int *s = L->src_rects + 4 * p->src, *r = L->req_rects + 4 * p->dst;
+            rp[k].src = (const double *) src_blks[p->src] +
+                        (long long) (p->srow - s[0]) * src_lds[p->src] + (p->scol - s[1]);
+            rp[k].dst = (double *) dst_blks[p->dst] +
+                        (long long) (p->srow - r[0]) * dst_lds[p->dst] + (p->scol - r[1]);
+            rp[k].lds = src_lds[p->src];
+            rp[k].ldd = dst_lds[p->dst];
+            rp[k].len = p->ncol;
+            rp[k].runs = p->nrow;
+        }
+        int rc = ca3dmm_copy_runs_launch(rp, L->npiece, st);
+        if (rc) return rc;
+        if (!stream) CA3DMM_CUDA_TRY(cudaStreamSynchronize(st));
+        return CA3DMM_OK;
+    }
     /* the staging is rewritten below: the previous exec's upload must be done */
     CA3DMM_CUDA_TRY(cudaStreamSynchronize(st));
     for (int k = 0; k < L->npiece; k++) {
