@@ -117,6 +117,7 @@ typedef struct {
                                      (env CA3DMM_CRT_BAND, default 32 -- measured best at
                                      8000^3; 0: all tile rows in one band) */
     int crt_band_env;             /* crt_band as the environment set it */
+    int crt_plan_band;            /* the band of the uploaded plan's work list */
     int crt_overlap;              /* device exec: reconstruct band b beside the GEMM of band b + 1
                                      (env CA3DMM_CRT_OVERLAP, default 1) */
     int crt_overlap_blocks;       /* reconstruction blocks per SM beside the GEMM (1 or 2) */
@@ -1237,6 +1238,7 @@ static int plan_upload(ca3dmm_engine_p e, const void *A, int ldA, const void *B,
              * the tile columns stream through */
             g->band = pl->upload_for_host ? e->raster
                                           : (pl->crt_band > 0 ? pl->crt_band : (e->m + 127) / 128);
+            pl->crt_plan_band = g->band;
             g->tile_n = pl->crt_tile_n;
         }
         rc = ca3dmm_crt_plan_encode(&pl->crt, e->crt_moduli, ns, pl->cb, pl->cs, ns, pl->cb + ns,
@@ -1342,7 +1344,7 @@ static int crt_overlapped_gemm(ca3dmm_engine_p e, plan_t *pl, int *status_d, cud
     *rc_out = CA3DMM_OK;
     if (!pl->crt_overlap || pl->crt_nsl != 1 || pl->upload_for_host || e->m <= 0) return 0;
     const int tiles_m = (e->m + 127) / 128;
-    const int band = pl->crt_band > 0 ? pl->crt_band : tiles_m;
+    const int band = pl->crt_plan_band > 0 ? pl->crt_plan_band : tiles_m;
     int per = band, nb = (tiles_m + band - 1) / band;
     while (nb > CRT_MAX_BANDS) {              /* several work-list bands per launch */
         per += band;
@@ -1482,8 +1484,9 @@ static int exec_device(ca3dmm_engine_p e, const void *src_A, int ldA, const void
         rc = ca3dmm_reduce_slabs_launch((const double *) (w + pl->off_slab),
                                         (long long) pl->slab_stride, pl->slab_ld, nred, e->m,
                                         e->n, out, ldo, st);
-    if (!rc && pl->sym && !crt)      /* the modular mode computes all of C */
-        rc = ca3dmm_mirror_upper_launch(out, ldo, e->m, st);
+    /* B^T B: the modular mode computes the upper triangle always (the lower one
+     * has the same bits), the others when asked to */
+    if (!rc && (pl->sym || (crt && e->is_BTB))) rc = ca3dmm_mirror_upper_launch(out, ldo, e->m, st);
     nvtxRangePop();
     if (rc) return rc;
     const int sums = crt || nred > 1 || pl->sym, copies = pl->has_dst && !whole;
@@ -1903,7 +1906,7 @@ static int hx_btb_slabs(ca3dmm_engine_p e, struct host_exec *x, const void *B_h,
     const int nred = kp * ks;
     rc = ca3dmm_reduce_slabs_launch((const double *) (w + pl->off_slab), (long long) pl->slab_stride,
                                     pl->slab_ld, nred, e->m, e->n, x->dC, x->ldc, st);
-    if (!rc && pl->sym) rc = ca3dmm_mirror_upper_launch(x->dC, x->ldc, e->m, st);
+    if (!rc && (pl->sym || crt)) rc = ca3dmm_mirror_upper_launch(x->dC, x->ldc, e->m, st);
     if (rc) return rc;
     CA3DMM_CUDA_TRY(cudaMemcpy2DAsync(C_h, sizeof(double) * (size_t) ldC, x->dC,
                                       sizeof(double) * (size_t) x->ldc, sizeof(double) * (size_t) e->m,

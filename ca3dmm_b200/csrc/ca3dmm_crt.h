@@ -35,7 +35,9 @@ extern "C" {
  * m x n over the blocks' k range (the same for both).  band: 128-row tile
  * rows per band of the GEMM's work list (0 = 8); within a band the moduli
  * run one after the other over the band's tiles, so a band of output rows is
- * one contiguous range of work items. */
+ * one contiguous range of work items.  A group whose A block aliases its B block
+ * (B^T B; m = n) computes the entries of C on and above the diagonal: the caller
+ * mirrors them (ca3dmm_mirror_upper_launch, after any slab sum). */
 typedef struct {
     int a_blk, b_blk;
     double *C;
@@ -52,7 +54,7 @@ typedef struct {
     int kc_tiles[2], rc_tiles[2];
     int p_min, p_max;     /* integer widths of the groups */
     long long n_exp;
-    long long recon_items;  /* reconstruction items (4 rows x 1 column) over every group */
+    long long recon_items;  /* reconstruction items (32 rows x 8 columns) over every group */
     int group_m, group_n;   /* the group's size when the plan has one group */
     int tile_n;             /* GEMM tile columns of every group */
     void *dev_plan;

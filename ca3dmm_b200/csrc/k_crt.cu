@@ -278,7 +278,8 @@ struct CrtGroup {
     double *C;
     long long ldc;
     int m, n, k;
-    int a_desc, b_desc, a_from_b;   // a_from_b: A tile tm is half tm % 2 of the B block's tile tm / 2
+    int a_desc, b_desc, a_from_b;   // a_from_b (B^T B): A tile tm is half tm % 2 of the B block's tile
+                                    // tm / 2, and only C's upper block triangle is computed
     int tiles_m, tiles_n, item_begin, band;
     int tile_n, pad_;               // GEMM tile columns (128 or 256; the same in every group)
     long long rc_begin;             // first reconstruction item (32 rows x 8 columns) of the group
@@ -317,13 +318,43 @@ __device__ __forceinline__ int find_group(const int *sb, const CrtGroup *g, int 
     return lo;
 }
 
+// Tiles of a group's first x tile rows.  B^T B (op(A) = B^T has B's own residues,
+// so C is symmetric, bit for bit: the same integers and the same scaling): only
+// the tiles that reach the diagonal or lie above it, columns tn0 .. tiles_n - 1 of
+// tile row y with tn0 = 128 y / tile_n rounded down.  The caller mirrors C.
+__host__ __device__ inline int tiles_before(const CrtGroup &G, int x)
+{
+    if (!G.a_from_b) return x * G.tiles_n;
+    if (x <= 0) return 0;
+    return x * G.tiles_n - (G.tile_n == 128 ? x * (x - 1) / 2 : (x - 1) * (x - 1) / 4);
+}
+
 // work item -> (modulus t, tile row tm, tile column tn) of its group: bands of
 // `band` tile rows; inside a band the moduli in turn, each over the band's
-// tiles with the tile row fastest
+// tiles with the tile row fastest (B^T B: tile row by tile row)
 __device__ __forceinline__ void item_decode(const CrtGroup &G, int nmod, int item, int &t, int &tm,
                                             int &tn)
 {
     const int local = item - G.item_begin;
+    if (G.a_from_b) {
+        int row = 0, next = min(G.band, G.tiles_m);
+        while (next < G.tiles_m && local >= nmod * tiles_before(G, next)) {
+            row = next;
+            next = min(next + G.band, G.tiles_m);
+        }
+        const int before = tiles_before(G, row), per_t = tiles_before(G, next) - before;
+        const int rem = local - nmod * before;
+        t = rem / per_t;
+        int r = rem - t * per_t;
+        for (tm = row;; ++tm) {
+            const int tn0 = tm * CBM / G.tile_n, w = G.tiles_n - tn0;
+            if (r < w) {
+                tn = tn0 + r;
+                return;
+            }
+            r -= w;
+        }
+    }
     const int full = nmod * G.band * G.tiles_n;
     const int b = local / full;
     const int rem = local - b * full;
@@ -567,6 +598,12 @@ crt_gemm_kernel(const CrtGroup *__restrict__ groups, int ngroup, int nmod,
                 I.plane = work + G.pl_off + ((long long) tm * nmod + t) * PL_BLOCK +
                           (tn * TN >> 5) * I.pl_col;
                 I.ncols = tile_cols(G, tn, TN);
+                if (G.a_from_b && TN == CBN && (tm & 1) && tn == tm >> 1) {
+                    // the tile's first 128 columns lie below the diagonal
+                    I.qb += CBM * CKB;
+                    I.plane += (CBM / 32) * I.pl_col;
+                    I.ncols -= CBM;
+                }
                 I.nkb = G.nkb;
                 I.k = G.k;
                 I.t = t;
@@ -868,6 +905,7 @@ crt_reconstruct_kernel(const CrtGroup *__restrict__ groups, int g0, int g1, int 
                                    : (int) ((unsigned int) local / (unsigned int) nq);
         const int i0 = rb + RC_ROWS * (int) (local - (long long) jp * nq), j0 = PL_COLS * jp;
         const int i = i0 + lane, ncol = min(PL_COLS, G.n - j0);
+        if (G.a_from_b && j0 + ncol <= i0) continue;          // below the diagonal: mirrored
         const unsigned char *pl = work + G.pl_off +
                                   ((long long) (j0 >> 5) * G.tiles_m + i0 / CBM) * (N * PL_BLOCK) +
                                   (j0 & 31) * CBM + (i & (CBM - 1)) * PL_COLS;
@@ -1061,6 +1099,7 @@ extern "C" int ca3dmm_crt_plan_encode(ca3dmm_crt_plan_t *pl, int nmod, int nA,
         o.a_desc = al >= 0 ? nA + al : G[g].a_blk;
         o.b_desc = nA + G[g].b_blk;
         o.a_from_b = al >= 0 ? 1 : 0;
+        if (al >= 0 && (o.m != o.n || al != G[g].b_blk)) return CA3DMM_EINVAL;
         o.tiles_m = (o.m > 0 && o.n > 0) ? (o.m + CBM - 1) / CBM : 0;
         o.tile_n = G[g].tile_n == 128 ? 128 : CBN;
         if (o.tile_n != (G[0].tile_n == 128 ? 128 : CBN)) return CA3DMM_EINVAL;
@@ -1079,7 +1118,7 @@ extern "C" int ca3dmm_crt_plan_encode(ca3dmm_crt_plan_t *pl, int nmod, int nA,
         o.qb_tstride = db.t_stride;
         o.pl_off = (long long) qoff;
         qoff += align256((size_t) nmod * crt_plane_bytes(o.m, o.n));
-        items += nmod * o.tiles_m * o.tiles_n;
+        items += nmod * tiles_before(o, o.tiles_m);
         if (o.tiles_m > 0) {
             pmin = o.P < pmin ? o.P : pmin;
             pmax = o.P > pmax ? o.P : pmax;
@@ -1111,8 +1150,8 @@ extern "C" int ca3dmm_crt_group_items(const void *host_plan, int g, int tile_lo,
     if (hi <= lo) { *begin = o.item_begin; *count = 0; return CA3DMM_OK; }
     // a range of whole bands: tile_lo a multiple of the band (or the group's start)
     if (lo % o.band || (hi % o.band && hi != o.tiles_m)) return CA3DMM_EINVAL;
-    *begin = o.item_begin + (lo / o.band) * hd->nmod * o.band * o.tiles_n;
-    *count = hd->nmod * (hi - lo) * o.tiles_n;
+    *begin = o.item_begin + hd->nmod * tiles_before(o, lo);
+    *count = hd->nmod * (tiles_before(o, hi) - tiles_before(o, lo));
     return CA3DMM_OK;
 }
 
