@@ -584,7 +584,7 @@ dgemm_dmma_segments(const __grid_constant__ CUtensorMap map_a,
         int left = sg.kt1 - sg.kt0;
         // the warps of rows 64 .. 127 start with half a chunk: of an SM quarter's two
         // warps one keeps the tensor pipe busy while the other moves its sums
-        int len = warp >= CONSUMER_WARPS / 2 ? chunk / 2 : chunk;
+        int len = warp >= CONSUMER_WARPS / 2 && left > chunk ? chunk / 2 : chunk;
         bool totalled = false;
         for (;;) {
 #pragma unroll
@@ -946,7 +946,11 @@ extern "C" int ca3dmm_dgemm_launch_ranges_tn(const void *dev_plan, int nprob,
 // for the cut tiles).  Whole calls: 194 -> 124 and 629 -> 591 us; 1501 x 2003 x
 // 3001 with both operands transposed 747 -> 694; 200 x 150 x 300 77 -> 71.  A product of few blocks is not spread over all SMs: the
 // partials read back by the last CTA of a tile grow with the parts, so the
-// number of CTAs is at most sqrt(2.5 T T K).
+// number of CTAs is at most sqrt(2.5 T T K).  From k = 512 on a share is at least
+// one chunk: chains of 256 k keep the error of this path, which the accuracy guard
+// of the tuner and the split-precision modes are held against, close below that of
+// the sub-slabs of 512 k and more (a 768^3 product in shares of 187 k would be half
+// as far off as its seven INT8 slices were meant to match).
 namespace {
 constexpr int SEG_SMS = 148, SEG_MAX_TILES = 16 * SEG_SMS, SEG_RASTER = 8;
 
@@ -968,6 +972,8 @@ bool seg_shape(int m, int n, int k, SegShape &s)
     double g = std::sqrt(2.5 * (double) s.T * (double) s.T * (double) s.K);
     if (g > SEG_SMS) g = SEG_SMS;
     if (g > (double) (s.T * s.K)) g = (double) (s.T * s.K);
+    if (s.K >= 2 * CA3DMM_DGEMM_CHUNK && g > (double) (s.T * s.K / CA3DMM_DGEMM_CHUNK))
+        g = (double) (s.T * s.K / CA3DMM_DGEMM_CHUNK);
     s.grid = g < 1.0 ? 1 : (int) g;
     const double parts = s.T >= s.grid ? 2.0 : (double) s.grid / (double) s.T + 1.0;
     const double seg = (double) s.T * (double) s.K / s.grid + 1.1 + 0.4 * parts;
