@@ -4,7 +4,8 @@
 //
 // Replaces the reference's per-Cannon-step cublasDgemm + stream sync
 // (src/cannon.c:410-418, :651-676; src/cuda_proxy.cu:211-230).  All virtual
-// ranks' cuboid GEMMs of one ca3dmm exec run in this single launch.
+// ranks' cuboid GEMMs of one ca3dmm exec run in this single launch -- or, for a
+// product of few tiles, as k segments of its tiles shared out evenly (below).
 //
 // Layout (per stage, 32 KiB for 128-column tiles or 24 KiB for 64-column
 // ones, 1024-byte aligned):
@@ -943,14 +944,15 @@ extern "C" int ca3dmm_dgemm_launch_ranges_tn(const void *dev_plan, int nprob,
 // back.  At 1000^3 (T = 64, K = 63) that is 63 against 31: measured 148 us
 // against 70; at 2048^3 the sub-slabs of 512 k and their sum took 574 us, the
 // segments 523 (2.3 us per block of the 93 % busy tensor pipe, 3 us to start, 3
-// for the cut tiles).  Whole calls: 194 -> 124 and 629 -> 591 us; 1501 x 2003 x
-// 3001 with both operands transposed 747 -> 694; 200 x 150 x 300 77 -> 71.  A product of few blocks is not spread over all SMs: the
-// partials read back by the last CTA of a tile grow with the parts, so the
-// number of CTAs is at most sqrt(2.5 T T K).  From k = 512 on a share is at least
-// one chunk: chains of 256 k keep the error of this path, which the accuracy guard
-// of the tuner and the split-precision modes are held against, close below that of
-// the sub-slabs of 512 k and more (a 768^3 product in shares of 187 k would be half
-// as far off as its seven INT8 slices were meant to match).
+// for the cut tiles).
+// A product of few blocks is not spread over all SMs: the partials read back by
+// the last CTA of a tile grow with the parts, so the number of CTAs is at most
+// sqrt(2.5 T T K).  From k = 512 on a share is at least one chunk: chains of 256 k
+// keep the error of this path, which the accuracy guard of the tuner and the
+// split-precision modes are held against, close below that of the sub-slabs of 512
+// k and more (in shares of 187 k a 768^3 product is off by 4.0e-16, less than the
+// seven INT8 slices that are to match it, 4.5e-16).  The price at 768^3: 16 blocks
+// per CTA instead of 12.
 namespace {
 constexpr int SEG_SMS = 148, SEG_MAX_TILES = 16 * SEG_SMS, SEG_RASTER = 8;
 
