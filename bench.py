@@ -830,6 +830,9 @@ def main():
     if head == "crt":
         nm = eng.s.crt_moduli
         ops = flops * nm                        # one INT8 product per modulus
+        if btb:                                 # of which the upper triangle of 128-blocks runs
+            t = (n + 127) // 128
+            ops *= (t + 1) / (2.0 * t)
         roof = {"bound": "tensor", "kernel": "crt_gemm_kernel",
                 "achieved": ops / (gemm_ms * 1e-3) / 1e12, "peak": int8_peak, "unit": "TFLOP/s",
                 "peak_source": int8_src, "traffic": traffic.get("crt_gemm_kernel")}
