@@ -268,10 +268,12 @@ static void plan_layout(ca3dmm_engine_p e, plan_t *pl)
     pl->off_slab = off;
     int nslab = e->kp * pl->ksplit;          /* plain mode's sub-slabs; split mode uses kp of them */
     if (pl->crt_nsl > nslab) nslab = pl->crt_nsl;
-    if (pl->seg_plan && e->gemm_mode == CA3DMM_GEMM_PLAIN)
-        off = align_up(off + ca3dmm_dgemm_segments_ws_bytes(e->m, e->n, e->k));
-    else if (nslab > 1)
-        off = align_up(off + sizeof(double) * pl->slab_stride * (size_t) nslab);
+    /* the partials of cut tiles too, in every mode: a buffer sized in one mode must
+     * not be too small for the plain one */
+    size_t slab_bytes = nslab > 1 ? sizeof(double) * pl->slab_stride * (size_t) nslab : 0;
+    if (pl->seg_plan && slab_bytes < ca3dmm_dgemm_segments_ws_bytes(e->m, e->n, e->k))
+        slab_bytes = ca3dmm_dgemm_segments_ws_bytes(e->m, e->n, e->k);
+    off = align_up(off + slab_bytes);
     GUARD_BAND(off);
     pl->off_cout = off;
     off = align_up(off + sizeof(double) * (size_t) e->m * (size_t) e->n);

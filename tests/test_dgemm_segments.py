@@ -105,3 +105,28 @@ def test_segments_against_double_double(cuda, monkeypatch, m, n, k, ta, tb, p):
         assert np.all(d <= k * 2.0 ** -53 * ab)
         err[merge] = np.sqrt(np.mean((d / ab) ** 2))
     assert err["1"] <= 1.1 * err["0"] + 3 * 2.0 ** -53 / np.sqrt(k), err
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k,p", [(300, 200, 400, 1), (1000, 900, 800, 4)])
+def test_buffer_sized_in_split_mode_serves_plain(cuda, monkeypatch, m, n, k, p):
+    """A caller's work buffer of the size asked for in a split-precision mode
+    holds the plain mode's layout."""
+    import torch
+    from tests._util import dev_zeros, from_dev, to_dev
+    A, B = np.random.default_rng(1).standard_normal((m, k)), np.random.default_rng(2).standard_normal((k, n))
+    dA, lda = to_dev(A)
+    dB, ldb = to_dev(B)
+    outs = []
+    for mode in ("0", "1", "2"):
+        monkeypatch.setenv("CA3DMM_GEMM_MODE", mode)
+        e = cb.Ca3dmmEngine(m, n, k, 0, 0, p=p, caller_workbuf=True)
+        assert e.ok
+        w = torch.empty(e.workbuf_bytes + 256, dtype=torch.uint8, device="cuda")
+        e.attach_workbuf((w.data_ptr() + 255) // 256 * 256)
+        assert e.set_gemm_mode(cb.GEMM_PLAIN) == 0
+        dC = dev_zeros(m * n)
+        assert e.exec(dA, lda, dB, ldb, dC, m) == 0
+        outs.append(from_dev(dC, m, n))
+        e.free()
+    assert np.array_equal(outs[0], outs[1]) and np.array_equal(outs[0], outs[2])
