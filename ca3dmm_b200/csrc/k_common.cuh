@@ -121,6 +121,18 @@ CA3DMM_DEV bool mbar_wait_bounded(uint64_t *bar, uint32_t parity, volatile int *
     }
 }
 
+// The same wait made by all 32 lanes of a warp, with one result for all of them.
+// Each lane polls by itself, so near the limit one lane may give up while another
+// sees the phase complete; warp-wide instructions after the wait (mma.sync,
+// tcgen05.ld / .st / .wait, __syncwarp) need every lane, so either all go on or
+// none does.  The vote also brings the lanes together again after the loop's
+// several exits.
+CA3DMM_DEV bool mbar_wait_warp(uint64_t *bar, uint32_t parity, volatile int *abort, int *status,
+                               int code, uint64_t limit_ns)
+{
+    return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort, status, code, limit_ns));
+}
+
 // 2D tiled TMA load into shared memory, completing on `bar` (tx bytes).
 // The tensor map lives in global memory (64-byte aligned, written by the
 // host before the launch).

@@ -479,17 +479,15 @@ crt_gemm_kernel(const CrtGroup *__restrict__ groups, int ngroup, int nmod,
     __syncthreads();
     tc_fence_after();
 
-    auto item_wait = [&](uint32_t i, int code) -> bool {
-        return mbar_wait_bounded(&item_full[i % ITEM_RING], (i / ITEM_RING) & 1u, &abort_flag,
-                                 status, code, limit_ns);
-    };
     if (warp == 0) {
         // ------------------------------------------------------ producer
         if (lane == 0) {
             uint32_t it = 0, ii = 0;
             bool ok = true;
             for (int v = blockIdx.x; v < total_items && ok && !abort_flag; v += gridDim.x) {
-                if (!item_wait(ii, CA3DMM_DEV_TIMEOUT_PRODUCE)) break;
+                if (!mbar_wait_bounded(&item_full[ii % ITEM_RING], (ii / ITEM_RING) & 1u, &abort_flag,
+                                       status, CA3DMM_DEV_TIMEOUT_PRODUCE, limit_ns))
+                    break;
                 const CrtItem &I = ring[ii % ITEM_RING];
                 const unsigned char *qa = I.qa, *qb = I.qb;
                 const int a_step = I.a_step, nkb = I.nkb;
@@ -524,7 +522,8 @@ crt_gemm_kernel(const CrtGroup *__restrict__ groups, int ngroup, int nmod,
             uint32_t it = 0, ai = 0;
             bool ok = true;
             for (int v = blockIdx.x; v < total_items && ok; v += gridDim.x, ++ai) {
-                if (!item_wait(ai, CA3DMM_DEV_TIMEOUT_ACCUM)) {
+                if (!mbar_wait_bounded(&item_full[ai % ITEM_RING], (ai / ITEM_RING) & 1u, &abort_flag,
+                                       status, CA3DMM_DEV_TIMEOUT_ACCUM, limit_ns)) {
                     ok = false;
                     break;
                 }
@@ -617,7 +616,9 @@ crt_gemm_kernel(const CrtGroup *__restrict__ groups, int ngroup, int nmod,
         const int h = (warp - 3) >> 2;                // accumulator columns TN/2 h .. TN/2 (h + 1) - 1
         uint32_t ai = 0;
         for (int v = blockIdx.x; v < total_items; v += gridDim.x, ++ai) {
-            if (!item_wait(ai, CA3DMM_DEV_TIMEOUT_EPI)) break;
+            if (!mbar_wait_warp(&item_full[ai % ITEM_RING], (ai / ITEM_RING) & 1u, &abort_flag,
+                                status, CA3DMM_DEV_TIMEOUT_EPI, limit_ns))
+                break;
             const CrtItem &I = ring[ai % ITEM_RING];
             const EpiConst mc = kEpi.e[nmod][I.t];
             unsigned char *plane = I.plane + (q * 32 + lane) * PL_COLS;
@@ -626,8 +627,8 @@ crt_gemm_kernel(const CrtGroup *__restrict__ groups, int ngroup, int nmod,
             __syncwarp();
             if (lane == 0) mbar_arrive(&item_empty[ai % ITEM_RING]);
             const uint32_t buf = ai & 1u;
-            if (!mbar_wait_bounded(&acc_full[buf], (ai >> 1) & 1u, &abort_flag, status,
-                                   CA3DMM_DEV_TIMEOUT_EPI, limit_ns))
+            if (!mbar_wait_warp(&acc_full[buf], (ai >> 1) & 1u, &abort_flag, status,
+                                CA3DMM_DEV_TIMEOUT_EPI, limit_ns))
                 break;
             tc_fence_after();
             // C's residues lie [column / 32][tile row][modulus][column % 32 / 8][128 rows][8

@@ -207,8 +207,8 @@ __device__ __forceinline__ bool k_loop(const uint8_t *smem, uint64_t *full, uint
     constexpr int MI = T::MI;
     for (int kt = 0; kt < ktiles; ++kt, ++it) {
         const uint32_t stage = it % T::STAGES, phase = (it / T::STAGES) & 1u;
-        if (!mbar_wait_bounded(&full[stage], phase, abort_flag, status,
-                               CA3DMM_DEV_TIMEOUT_CONSUME, limit_ns))
+        if (!mbar_wait_warp(&full[stage], phase, abort_flag, status, CA3DMM_DEV_TIMEOUT_CONSUME,
+                            limit_ns))
             return false;
         const uint8_t *sA = smem + stage * T::STAGE_BYTES;
         const uint8_t *sB = sA + A_BYTES;
@@ -263,8 +263,11 @@ __device__ __forceinline__ bool k_loop(const uint8_t *smem, uint64_t *full, uint
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[stage]);
-        if (producer && !issue_one()) return false;
+        // a refill that gives up has raised the abort flag: the wait for the missing
+        // load ends the loop, for the whole warp
+        if (producer) issue_one();
     }
+    __syncwarp();
     return true;
 }
 
@@ -630,20 +633,17 @@ dgemm_dmma_segments(const __grid_constant__ CUtensorMap map_a,
             if (lane == 0) mbar_arrive(&fix_bar[0]);
             const uint32_t ph = nfix & 1u;
             ++nfix;
-            if (producer) {
-                if (!mbar_wait_bounded(&fix_bar[0], ph, &abort_flag, status,
-                                       CA3DMM_DEV_TIMEOUT_ACCUM, limit_ns)) {
-                    ok = false;
-                } else {
-                    const bool last = atomicAdd(counters + sg.counter, 1) == nparts - 1;
-                    if (last) counters[sg.counter] = 0;      // for the next launch
-                    __threadfence();
-                    last_part = last;
-                    mbar_arrive(&fix_bar[1]);
-                }
+            // (a wait that fails here has raised the abort flag, which ends the next one)
+            if (producer && mbar_wait_bounded(&fix_bar[0], ph, &abort_flag, status,
+                                              CA3DMM_DEV_TIMEOUT_ACCUM, limit_ns)) {
+                const bool last = atomicAdd(counters + sg.counter, 1) == nparts - 1;
+                if (last) counters[sg.counter] = 0;      // for the next launch
+                __threadfence();
+                last_part = last;
+                mbar_arrive(&fix_bar[1]);
             }
-            ok = ok && mbar_wait_bounded(&fix_bar[1], ph, &abort_flag, status,
-                                         CA3DMM_DEV_TIMEOUT_ACCUM, limit_ns);
+            ok = mbar_wait_warp(&fix_bar[1], ph, &abort_flag, status, CA3DMM_DEV_TIMEOUT_ACCUM,
+                                limit_ns);
             if (!ok) break;
             if (!last_part) continue;
             __threadfence();
@@ -689,6 +689,7 @@ dgemm_dmma_segments(const __grid_constant__ CUtensorMap map_a,
             }
         }
     }
+    __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 1) {

@@ -435,8 +435,8 @@ oz_gemm_kernel(const OzGroup *__restrict__ groups, const OzUnit *__restrict__ un
             for (int j = 0; j < 32; ++j) acc[j] = 0.0;
             const int nch = nchunks(p.nkb, kb_per_chunk);
             for (int ch = 0; ch < nch; ++ch, ++ci) {
-                if (!mbar_wait_bounded(acc_full, ci & 1u, &abort_flag, status,
-                                       CA3DMM_DEV_TIMEOUT_EPI, limit_ns)) {
+                if (!mbar_wait_warp(acc_full, ci & 1u, &abort_flag, status, CA3DMM_DEV_TIMEOUT_EPI,
+                                    limit_ns)) {
                     ok = false;
                     break;
                 }

@@ -139,8 +139,8 @@ pack_transpose_tma_kernel(const CUtensorMap *__restrict__ tmaps,
     bool ok = true;
     for (int i = 0; i < mine && ok; ++i) {
         const int s = i % TT_STAGES;
-        if (!mbar_wait_bounded(&full[s], (uint32_t) (i / TT_STAGES) & 1u, &abort_flag, status,
-                               CA3DMM_DEV_TIMEOUT_CONSUME, limit_ns)) {
+        if (!mbar_wait_warp(&full[s], (uint32_t) (i / TT_STAGES) & 1u, &abort_flag, status,
+                            CA3DMM_DEV_TIMEOUT_CONSUME, limit_ns)) {
             ok = false;
             break;
         }
