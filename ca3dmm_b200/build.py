@@ -22,7 +22,7 @@ C_SOURCES = ["vcomm.c", "partition.c", "dev_type.c", "mat_redist.c", "cannon.c",
              "grouped.c", "autotune.c", "dist.c", "transport.c"]
 CU_SOURCES = ["k_dgemm.cu", "k_pack.cu", "k_ozaki.cu", "k_crt.cu", "k_noalloc.cu", "k_mlp.cu",
               "k_tune_guard.cu"]
-HEADERS = ["ca3dmm_kernels.h", "ca3dmm_ozaki.h", "ca3dmm_crt.h", "ca3dmm_util.h", "k_common.cuh",
+HEADERS = ["ca3dmm_kernels.h", "ca3dmm_ozaki.h", "ca3dmm_crt.h", "ca3dmm_util.h", "ca3dmm_stage.h", "k_common.cuh",
            "k_split.cuh", "ca3dmm_tune_guard.h", "ca3dmm_tune_internal.h"]
 EXAMPLES = ["example_cholesky_qr", "example_ab", "example_btb", "example_ab_dist"]
 

@@ -25,6 +25,7 @@
 #include <cuda_runtime_api.h>
 #include <nvtx3/nvToolsExt.h>
 #include "ca3dmm_util.h"
+#include "ca3dmm_stage.h"
 #include "ca3dmm_kernels.h"
 #include "ca3dmm_ozaki.h"
 #include "ca3dmm_crt.h"
@@ -69,9 +70,8 @@ typedef struct {
     size_t gemm_plan_bytes, oz_plan_bytes, oz_bytes;
     long long slab_ld;        /* leading dimension of each C slab */
     size_t slab_stride;       /* elements between slabs */
-    /* pinned host staging for plan uploads */
-    void *stage;
     size_t stage_bytes;
+    ca3dmm_stage_t stage;         /* page-locked host staging of the plan uploads */
     /* the status words of every launch: page-locked host memory that the kernels
      * write where it lies (only when a bounded wait runs out or a guard band is
      * overwritten), so an exec needs no clearing before and no copy after it */
@@ -487,11 +487,9 @@ static int plan_build(ca3dmm_engine_p e)
  * that init itself makes no CUDA call (it only sizes the work buffer). */
 static int plan_cuda_init(plan_t *pl)
 {
-    if (pl->stage) return CA3DMM_OK;
-    if (cudaMallocHost(&pl->stage, pl->stage_bytes) != cudaSuccess) {
-        pl->stage = NULL;
-        return CA3DMM_ECUDA;
-    }
+    if (pl->stage.buf) return CA3DMM_OK;
+    int rc = ca3dmm_stage_create(&pl->stage, pl->stage_bytes);
+    if (rc) return rc;
     if (cudaMallocHost((void **) &pl->status_h, 64) != cudaSuccess) {
         pl->status_h = NULL;
         return CA3DMM_ECUDA;
@@ -535,7 +533,7 @@ static void plan_free(plan_t *pl)
         }
         free(x);
     }
-    if (pl->stage) cudaFreeHost(pl->stage);
+    ca3dmm_stage_free(&pl->stage);
     if (pl->status_h) cudaFreeHost(pl->status_h);
     if (pl->events_ok)
         for (int i = 0; i < 5; i++) cudaEventDestroy(pl->ev[i]);
@@ -988,7 +986,10 @@ static int plan_upload(ca3dmm_engine_p e, const void *A, int ldA, const void *B,
                        void *dst, int ldC, cudaStream_t st)
 {
     plan_t *pl = (plan_t *) e->impl;
-    char *w = (char *) e->workbuf_d, *h = (char *) pl->stage;
+    int rc = ca3dmm_stage_begin(&pl->stage);
+    if (rc) return rc;
+    pl->plan_valid = 0;
+    char *w = (char *) e->workbuf_d, *h = (char *) pl->stage.buf;
     /* An operand block whose address and leading dimension suit the GEMM's
      * tensor maps (16-byte aligned start, even ld) is read in place: op(B)
      * untransposed (K-major), op(A) untransposed (M-major) or transposed
@@ -1136,8 +1137,8 @@ static int plan_upload(ca3dmm_engine_p e, const void *A, int ldA, const void *B,
             q->a_kmajor = pl->a_kmajor;
         }
     }
-    int rc = ca3dmm_dgemm_plan_encode_tn(gd, pl->ngroup * ks, h + pl->off_gemm, &pl->gemm_tiles,
-                                         pl->plain_tile_n);
+    rc = ca3dmm_dgemm_plan_encode_tn(gd, pl->ngroup * ks, h + pl->off_gemm, &pl->gemm_tiles,
+                                     pl->plain_tile_n);
     if (rc) return rc;
     if (seg) {
         const int mx = ca3dmm_dgemm_segments_max(e->m, e->n, e->k);
@@ -1250,12 +1251,13 @@ static int plan_upload(ca3dmm_engine_p e, const void *A, int ldA, const void *B,
         e->crt_bits = pl->crt.p_min;
     }
     memset(h + pl->off_counters, 0, COUNTER_BYTES);
-    CA3DMM_CUDA_TRY(cudaMemcpyAsync(w, h, pl->stage_bytes, cudaMemcpyHostToDevice, st));
+    rc = ca3dmm_stage_upload(&pl->stage, w, st);
+    if (rc) return rc;
     for (int i = 0; i < pl->ncanary; i++)
         CA3DMM_CUDA_TRY(cudaMemsetAsync(w + pl->canary[i], CANARY_BYTE, CANARY_BYTES, st));
     pl->c_A = A; pl->c_B = B; pl->c_ldA = ldA; pl->c_ldB = ldB;
     pl->c_dst = dst; pl->c_ldC = ldC;
-    pl->plan_valid = 1;
+    pl->plan_valid = !pl->stage.any_graph;
     return CA3DMM_OK;
 }
 
@@ -1286,7 +1288,7 @@ static int launch_segments(ca3dmm_engine_p e, const ca3dmm_tile_ranges_t *rg, cu
     if (!rg) sg += pl->seg_bytes / (2 * sizeof(*sg));
     const int lo = rg ? rg->begin[0] : 0, hi = rg ? lo + rg->len[0] : pl->nseg;
     return ca3dmm_dgemm_launch_segments(
-        (const char *) pl->stage + pl->off_gemm, pl->ngroup * pl->ksplit, sg,
+        (const char *) pl->stage.buf + pl->off_gemm, pl->ngroup * pl->ksplit, sg,
         rg ? NULL : pl->seg_begin, lo, hi, pl->seg_grid, pl->a_kmajor, w + pl->off_slab,
         (int *) (w + pl->off_counters), pl->status_h, 5.0, st,
         pl->plain_tile_n);
@@ -1360,7 +1362,7 @@ static int crt_overlapped_gemm(ca3dmm_engine_p e, plan_t *pl, int *status_d, cud
         cudaEventCreateWithFlags(&pl->ev_join, cudaEventDisableTiming);
         pl->aux_ok = 1;
     }
-    const char *hp = (const char *) pl->stage + pl->off_crtplan;
+    const char *hp = (const char *) pl->stage.buf + pl->off_crtplan;
     const int sms = ca3dmm_device_sm_count();
     int rc = CA3DMM_OK;
     for (int b = 0; b < nb && !rc; b++) {
@@ -1541,7 +1543,7 @@ void ca3dmm_engine_exec(ca3dmm_engine_p e, const void *src_A, const int ldA, con
         ERROR_PRINTF("ca3dmm_engine not initialized\n");
         return;
     }
-    if (e->workbuf_d == NULL || ((plan_t *) e->impl)->stage == NULL) {
+    if (e->workbuf_d == NULL || ((plan_t *) e->impl)->stage.buf == NULL) {
         ERROR_PRINTF("ca3dmm_engine has no device work buffer attached\n");
         e->last_error = CA3DMM_EINVAL;
         return;
@@ -1635,7 +1637,7 @@ static int hx_build_bands_crt(ca3dmm_engine_p e, struct host_exec *x, cudaStream
         if (cudaMallocHost(&x->desc_h, cap) != cudaSuccess) { x->desc_h = NULL; return 0; }
         if (cudaMalloc(&x->desc_d, cap) != cudaSuccess) { x->desc_d = NULL; return 0; }
     }
-    const char *hp = (const char *) pl->stage + pl->off_crtplan;
+    const char *hp = (const char *) pl->stage.buf + pl->off_crtplan;
     for (int r = 0; r < e->m; r += band_rows) {
         const int c = x->nband++;
         const int rend = r + band_rows < e->m ? r + band_rows : e->m;
@@ -1725,7 +1727,7 @@ static int hx_build_bands(ca3dmm_engine_p e, struct host_exec *x, cudaStream_t s
             const int row_lo = r / 128, nrow_t = band_rows / 128;
             if (seg) {
                 const ca3dmm_dgemm_seg_t *sg =
-                    (const ca3dmm_dgemm_seg_t *) ((char *) pl->stage + pl->off_seg);
+                    (const ca3dmm_dgemm_seg_t *) ((char *) pl->stage.buf + pl->off_seg);
                 int lo = 0, hi;
                 while (lo < pl->nseg && sg[lo].tm < row_lo) lo++;
                 for (hi = lo; hi < pl->nseg && sg[hi].tm < row_lo + nrow_t;) hi++;
@@ -1748,7 +1750,7 @@ static int hx_build_bands(ca3dmm_engine_p e, struct host_exec *x, cudaStream_t s
             char *dh = (char *) x->desc_h + (size_t) c * x->desc_stride;
             for (int tk = 0; tk < e->kp; tk++) blocks[tk] = tk * tmn + tm;
             if (ozaki) {
-                bad = ca3dmm_oz_encode_rows((char *) pl->stage + pl->off_ozplan, pl->ngroup, blocks,
+                bad = ca3dmm_oz_encode_rows((char *) pl->stage.buf + pl->off_ozplan, pl->ngroup, blocks,
                                             e->kp, r, rend, dh, x->ntile[c]);
             } else {
                 ca3dmm_pack_desc_t *pd = (ca3dmm_pack_desc_t *) dh;
@@ -1840,9 +1842,9 @@ static int hx_btb_slabs(ca3dmm_engine_p e, struct host_exec *x, const void *B_h,
         for (int j = 0; j < kp; j++) {
             char *dj = (char *) x->desc_h + (size_t) j * x->desc_stride;
             const int idx = crt ? pl->crt_nsl + j : pl->nA + j;
-            if (crt ? ca3dmm_crt_encode_blocks((char *) pl->stage + pl->off_crtplan, pl->crt_nsl,
+            if (crt ? ca3dmm_crt_encode_blocks((char *) pl->stage.buf + pl->off_crtplan, pl->crt_nsl,
                                                &idx, 1, dj, x->ntile[j])
-                    : ca3dmm_oz_encode_blocks((char *) pl->stage + pl->off_ozplan, pl->ngroup,
+                    : ca3dmm_oz_encode_blocks((char *) pl->stage.buf + pl->off_ozplan, pl->ngroup,
                                               &idx, 1, dj, x->ntile[j]))
                 return 1;
         }
@@ -1886,7 +1888,7 @@ static int hx_btb_slabs(ca3dmm_engine_p e, struct host_exec *x, const void *B_h,
         if (crt) {
             const void *dd = (const char *) x->desc_d + (size_t) j * x->desc_stride;
             int ib = 0, ic = 0;
-            rc = ca3dmm_crt_group_items((char *) pl->stage + pl->off_crtplan, j, 0, INT32_MAX, &ib,
+            rc = ca3dmm_crt_group_items((char *) pl->stage.buf + pl->off_crtplan, j, 0, INT32_MAX, &ib,
                                         &ic);
             rg.begin[0] = ib;
             rg.len[0] = ic;
@@ -2074,7 +2076,7 @@ int ca3dmm_engine_exec_host(ca3dmm_engine_p e, const void *A_h, int ldA, const v
         ERROR_PRINTF("ca3dmm_engine not initialized\n");
         return CA3DMM_EINVAL;
     }
-    if (e->workbuf_d == NULL || ((plan_t *) e->impl)->stage == NULL) {
+    if (e->workbuf_d == NULL || ((plan_t *) e->impl)->stage.buf == NULL) {
         ERROR_PRINTF("ca3dmm_engine has no device work buffer attached\n");
         e->last_error = CA3DMM_EINVAL;
         return CA3DMM_EINVAL;

@@ -6,6 +6,7 @@
 #include <string.h>
 #include <cuda_runtime_api.h>
 #include "ca3dmm_util.h"
+#include "ca3dmm_stage.h"
 #include "ca3dmm_kernels.h"
 #include "ca3dmm_ozaki.h"
 #include "ca3dmm_crt.h"
@@ -26,7 +27,7 @@ struct ca3dmm_grouped {
     size_t oz_bytes, crt_bytes, stage_bytes;
     void *workbuf_d;
     int alloc_workbuf;
-    void *stage;                  /* pinned host staging of the plan */
+    ca3dmm_stage_t stage;         /* page-locked host staging of the plan */
     int *status_h;
     cudaEvent_t ev[2];
     int events_ok;
@@ -81,7 +82,7 @@ void ca3dmm_grouped_free(ca3dmm_grouped_p *gp)
     free(g->lda_p); free(g->ldb_p); free(g->offA); free(g->offB);
     free(g->cA); free(g->cB); free(g->cC); free(g->cldA); free(g->cldB); free(g->cldC);
     free(g->gd); free(g->ob); free(g->os); free(g->og); free(g->cg);
-    if (g->stage) cudaFreeHost(g->stage);
+    ca3dmm_stage_free(&g->stage);
     if (g->status_h) cudaFreeHost(g->status_h);
     if (g->events_ok) { cudaEventDestroy(g->ev[0]); cudaEventDestroy(g->ev[1]); }
     if (g->alloc_workbuf && g->workbuf_d) cudaFree(g->workbuf_d);
@@ -214,8 +215,9 @@ int ca3dmm_grouped_attach_workbuf(ca3dmm_grouped_p g, void *workbuf_d)
 {
     if (!g || !workbuf_d || ((uintptr_t) workbuf_d & 255)) return CA3DMM_EINVAL;
     g->workbuf_d = workbuf_d;
-    if (!g->stage) {
-        CA3DMM_CUDA_TRY(cudaMallocHost(&g->stage, g->stage_bytes));
+    if (!g->stage.buf) {
+        const int rc = ca3dmm_stage_create(&g->stage, g->stage_bytes);
+        if (rc) return rc;
         CA3DMM_CUDA_TRY(cudaMallocHost((void **) &g->status_h, 64));
         memset(g->status_h, 0, 64);
         g->events_ok = cudaEventCreate(&g->ev[0]) == cudaSuccess &&
@@ -249,7 +251,10 @@ static int build_plan(ca3dmm_grouped_p g, const double *const *A, const int *ldA
                       const double *const *B, const int *ldB, double *const *C, const int *ldC,
                       cudaStream_t st)
 {
-    char *w = (char *) g->workbuf_d, *h = (char *) g->stage;
+    int rc = ca3dmm_stage_begin(&g->stage);
+    if (rc) return rc;
+    g->plan_valid = 0;
+    char *w = (char *) g->workbuf_d, *h = (char *) g->stage.buf;
     const int np = g->nprob;
     memset(h, 0, 64);
     if (g->mode == 0) {
@@ -297,7 +302,7 @@ static int build_plan(ca3dmm_grouped_p g, const double *const *A, const int *ldA
         }
         g->tiles_A = ca3dmm_pack_tiles(pa, np);
         g->tiles_B = ca3dmm_pack_tiles(pb, np);
-        int rc = ca3dmm_dgemm_plan_encode(g->gd, np, h + g->off_gemm, &g->gemm_tiles);
+        rc = ca3dmm_dgemm_plan_encode(g->gd, np, h + g->off_gemm, &g->gemm_tiles);
         if (rc) return rc;
     } else {
         /* split precision: operand blocks read where they lie (absolute bases) */
@@ -310,7 +315,6 @@ static int build_plan(ca3dmm_grouped_p g, const double *const *A, const int *ldA
             g->ob[np + i].alias = -1;
             g->os[np + i].base = B[i]; g->os[np + i].ld = ldB[i]; g->os[np + i].trans = g->tb[i];
         }
-        int rc;
         if (g->mode == 2) {
             for (int j = 0; j < np; j++) {
                 const int i = g->order[j];
@@ -336,12 +340,13 @@ static int build_plan(ca3dmm_grouped_p g, const double *const *A, const int *ldA
         }
         if (rc) return rc;
     }
-    CA3DMM_CUDA_TRY(cudaMemcpyAsync(w, h, g->stage_bytes, cudaMemcpyHostToDevice, st));
+    rc = ca3dmm_stage_upload(&g->stage, w, st);
+    if (rc) return rc;
     for (int i = 0; i < np; i++) {
         g->cA[i] = A[i]; g->cB[i] = B[i]; g->cC[i] = C[i];
         g->cldA[i] = ldA[i]; g->cldB[i] = ldB[i]; g->cldC[i] = ldC[i];
     }
-    g->plan_valid = 1;
+    g->plan_valid = !g->stage.any_graph;
     return CA3DMM_OK;
 }
 

@@ -211,7 +211,13 @@ int ca3dmm_engine_guard_bands(ca3dmm_engine_p engine, long long *offsets, int ma
 /* First error of the last call on this engine (0 = none). */
 int ca3dmm_engine_last_error(ca3dmm_engine_p engine);
 /* Run exec on `stream` (cudaStream_t); sync = 0 makes exec asynchronous and
- * CUDA-graph capturable (the statistics are then not updated). */
+ * CUDA-graph capturable (the statistics are then not updated).  Asynchronous
+ * execs of one engine run in the order of the calls when their streams are so
+ * ordered.  An exec whose arguments differ from the last one's first waits on
+ * the host until that one's plan has been copied to the device.  A captured exec
+ * whose arguments differ from the last one's carries its plan in the graph and
+ * may be replayed at any time; one with the last exec's arguments reads the plan
+ * in the work buffer: replay it before the engine is given other ones. */
 void ca3dmm_engine_set_stream(ca3dmm_engine_p engine, void *stream, int sync);
 /* Select the GEMM: CA3DMM_GEMM_PLAIN, CA3DMM_GEMM_OZAKI with `slices` INT8
  * slices per operand (2..8), CA3DMM_GEMM_CRT with `slices` moduli (8..18,

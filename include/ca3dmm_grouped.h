@@ -33,7 +33,8 @@ int ca3dmm_grouped_init(int nprob, const int *m, const int *n, const int *k, con
                         size_t *workbuf_bytes);
 int ca3dmm_grouped_attach_workbuf(ca3dmm_grouped_p g, void *workbuf_d);
 /* stream: cudaStream_t (NULL = legacy default); sync = 1 (default): exec
- * waits and checks the device status; 0: exec only enqueues. */
+ * waits and checks the device status; 0: exec only enqueues.  Changing
+ * arguments and captured execs: as ca3dmm_engine_set_stream says. */
 void ca3dmm_grouped_set_stream(ca3dmm_grouped_p g, void *stream, int sync);
 /* A[i]: op(A_i) source (m x k, or k x m when trans), ldA[i] its leading
  * dimension; likewise B; C[i] column-major m x n with ldC[i] >= m.  Device
