@@ -36,6 +36,7 @@
 #define CANARY_BYTES 256
 #define CANARY_BYTE 0xA5
 /* the k segments' counters (cut tiles: at most one per CTA boundary and half tile) */
+#define STATUS_ASYNC 8
 #define COUNTER_BYTES (2 * CA3DMM_DGEMM_SEG_CTAS * (int) sizeof(int))
 
 typedef struct {
@@ -74,8 +75,11 @@ typedef struct {
     ca3dmm_stage_t stage;         /* page-locked host staging of the plan uploads */
     /* the status words of every launch: page-locked host memory that the kernels
      * write where it lies (only when a bounded wait runs out or a guard band is
-     * overwritten), so an exec needs no clearing before and no copy after it */
-    int *status_h;
+     * overwritten), so an exec needs no clearing before and no copy after it.
+     * Asynchronous execs have words of their own (status_h + STATUS_ASYNC): the
+     * host clears a synchronous exec's while they may still run. */
+    int *status_h, *status_use;
+    int async_used;               /* an asynchronous exec was queued or captured, once */
     int counters_clean;           /* the k segments' counters are zero (the last exec ended well) */
     /* cached exec arguments the device plan was built for */
     int plan_valid, c_ldA, c_ldB, c_ldC;
@@ -495,6 +499,7 @@ static int plan_cuda_init(plan_t *pl)
         return CA3DMM_ECUDA;
     }
     memset(pl->status_h, 0, 64);
+    pl->status_use = pl->status_h;
     pl->events_ok = 1;
     for (int i = 0; i < 5; i++)
         if (cudaEventCreate(&pl->ev[i]) != cudaSuccess) pl->events_ok = 0;
@@ -1273,7 +1278,7 @@ static int launch_pack_side(ca3dmm_engine_p e, int which, const void *src, cudaS
     if (which ? pl->packB_tma : pl->packA_tma)
         return ca3dmm_pack_tma_launch(w + (which ? pl->off_tmapB : pl->off_tmapA),
                                       (const ca3dmm_pack_desc_t *) (w + off_desc), nd, tiles,
-                                      (double *) w, pl->status_h, 5.0, st);
+                                      (double *) w, pl->status_use, 5.0, st);
     return ca3dmm_pack_launch((const double *) src, (double *) w,
                               (const ca3dmm_pack_desc_t *) (w + off_desc), nd, tiles, st);
 }
@@ -1290,14 +1295,19 @@ static int launch_segments(ca3dmm_engine_p e, const ca3dmm_tile_ranges_t *rg, cu
     return ca3dmm_dgemm_launch_segments(
         (const char *) pl->stage.buf + pl->off_gemm, pl->ngroup * pl->ksplit, sg,
         rg ? NULL : pl->seg_begin, lo, hi, pl->seg_grid, pl->a_kmajor, w + pl->off_slab,
-        (int *) (w + pl->off_counters), pl->status_h, 5.0, st,
-        pl->plain_tile_n);
+        (int *) (w + pl->off_counters), pl->status_use, 5.0, st, pl->plain_tile_n);
 }
 
 /* The device status word after a call: 0, a bounded wait that ran out, or
- * an overwritten guard band (status[1] holds its index). */
+ * an overwritten guard band (status[1] holds its index).  What asynchronous
+ * execs left in theirs is printed; it is not this call's result. */
 static int device_status_error(const plan_t *pl)
 {
+    int *late = pl->status_h + STATUS_ASYNC;
+    if (late[0]) {
+        ERROR_PRINTF("Device status %d of an earlier asynchronous exec\n", late[0]);
+        late[0] = late[1] = 0;
+    }
     const int code = pl->status_h[0];
     if (code == 0) return CA3DMM_OK;
     if (code == 6) {
@@ -1312,11 +1322,11 @@ static int device_status_error(const plan_t *pl)
 }
 
 /* The k segments' launches leave their counters zero; clear them when the last
- * exec may not have ended (an asynchronous one, or one that failed), and always
- * in an asynchronous exec, which may be captured and replayed. */
+ * exec may not have ended well, in an asynchronous exec, and in every exec of an
+ * engine that had one: a graph may be replayed, and run out of time, unseen. */
 static int counters_clear(plan_t *pl, char *w, int sync, cudaStream_t st)
 {
-    if (!pl->seg_plan || (sync && pl->counters_clean)) return CA3DMM_OK;
+    if (!pl->seg_plan || (sync && pl->counters_clean && !pl->async_used)) return CA3DMM_OK;
     CA3DMM_CUDA_TRY(cudaMemsetAsync(w + pl->off_counters, 0, COUNTER_BYTES, st));
     return CA3DMM_OK;
 }
@@ -1423,7 +1433,9 @@ static int exec_device(ca3dmm_engine_p e, const void *src_A, int ldA, const void
         if (rc) return rc;
     }
     pl->counters_clean = 0;
+    pl->status_use = pl->status_h + (e->sync_exec ? 0 : STATUS_ASYNC);
     if (e->sync_exec) pl->status_h[0] = pl->status_h[1] = 0;
+    else pl->async_used = 1;
     /* an event (about 5 us each) only where a phase begins or ends: plain FP64
      * often neither packs nor sums, and a whole C needs no copy */
     const int timing = e->sync_exec && pl->events_ok;
@@ -1445,7 +1457,7 @@ static int exec_device(ca3dmm_engine_p e, const void *src_A, int ldA, const void
     nvtxRangePop();
     if (rc) return rc;
     if (timing && packs) cudaEventRecord(pl->ev[1], st);
-    int *status_d = pl->status_h;
+    int *status_d = pl->status_use;
     nvtxRangePushA("ca3dmm: GEMM (2D Cannon)");
     int crt_bands = 0;
     if (crt) {
@@ -1853,7 +1865,7 @@ static int hx_btb_slabs(ca3dmm_engine_p e, struct host_exec *x, const void *B_h,
         x->slab_built = 1;
     }
     char *w = (char *) e->workbuf_d;
-    int *status_d = pl->status_h;
+    int *status_d = pl->status_use = pl->status_h;
     status_d[0] = status_d[1] = 0;
     /* copies in: B slab by slab */
     for (int j = 0; j < kp; j++) {
@@ -1999,7 +2011,7 @@ static int exec_host(ca3dmm_engine_p e, const void *A_h, int ldA, const void *B_
         return CA3DMM_OK;
     }
     char *w = (char *) e->workbuf_d;
-    int *status_d = pl->status_h;
+    int *status_d = pl->status_use = pl->status_h;
     status_d[0] = status_d[1] = 0;
     rc = counters_clear(pl, w, 1, st);
     if (rc) return rc;

@@ -2,6 +2,8 @@
 behind work that still runs, between synchronous calls, captured before the engine
 ever ran, replayed between direct calls.  Every C has the bits of a synchronous
 call on an engine of its own."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -146,3 +148,39 @@ def test_grouped_execs_with_changing_operands(cuda, mode):
         assert g.exec(*sets[2]) == 0
         check((0, 2))
     del graph
+
+
+def test_asynchronous_failure_is_not_the_next_calls(cuda, monkeypatch, capfd):
+    """An asynchronous exec that finds a guard band overwritten reports it in its own
+    status word, printed by the next synchronous exec, which succeeds."""
+    import torch
+    monkeypatch.setenv("CA3DMM_CANARY", "1")
+    m, n, k = 300, 260, 700
+    dA, lda = to_dev(orc.gen_signed_exp(3, m, k))
+    dB, ldb = to_dev(orc.gen_signed_exp(4, k, n))
+    dC = dev_zeros(m * n)
+    e = cb.Ca3dmmEngine(m, n, k, 0, 0, p=2, caller_workbuf=True)
+    w = torch.zeros(e.workbuf_bytes + 256, dtype=torch.uint8, device="cuda")
+    base = (-w.data_ptr()) % 256
+    e.attach_workbuf(w.data_ptr() + base)
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    e.set_stream(s.cuda_stream, 1)
+    assert e.exec(dA, lda, dB, ldb, dC, m) == 0
+    off = (ctypes.c_longlong * 2)()
+    assert cb.lib().ca3dmm_engine_guard_bands(e.e, off, 2) > 1
+    band = w[base + off[1]:][:256]
+    with torch.cuda.stream(s):
+        torch.cuda._sleep(20_000_000)
+        kept = band.clone()
+        band.zero_()
+        e.set_stream(s.cuda_stream, 0)
+        assert e.exec(dA, lda, dB, ldb, dC, m) == 0
+        band.copy_(kept)
+    e.set_stream(s.cuda_stream, 1)
+    capfd.readouterr()
+    assert e.exec(dA, lda, dB, ldb, dC, m) == 0
+    assert "Device status 6 of an earlier asynchronous exec" in capfd.readouterr().err
+    assert e.exec(dA, lda, dB, ldb, dC, m) == 0
+    assert "earlier" not in capfd.readouterr().err
+    e.free()
