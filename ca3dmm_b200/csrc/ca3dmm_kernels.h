@@ -143,13 +143,15 @@ int ca3dmm_pack_launch(const double *src_base, double *dst_base,
 
 /* Copies of up to CA3DMM_MAX_RUN_PIECES blocks in one launch, stream-ordered, the
  * blocks passed as kernel arguments: `runs` runs of `len` contiguous elements,
- * lds / ldd elements apart.  CA3DMM_EINVAL above that number of blocks. */
+ * lds / ldd elements apart.  CA3DMM_EINVAL above that number of blocks; blocks that
+ * ca3dmm_copy_runs_items refuses are an error. */
 #define CA3DMM_MAX_RUN_PIECES 512
 typedef struct {
     const double *src;
     double *dst;
     int lds, ldd, len, runs;
 } ca3dmm_run_piece_t;
+long long ca3dmm_copy_runs_items(const ca3dmm_run_piece_t *pieces, int n);   /* -1: not one launch */
 int ca3dmm_copy_runs_launch(const ca3dmm_run_piece_t *pieces, int n, cudaStream_t stream);
 
 /* One column-major block copy dst[r + c*ldd] = src[r + c*lds] (rows x cols),

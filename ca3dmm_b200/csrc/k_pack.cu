@@ -16,6 +16,7 @@
 namespace {
 
 constexpr int PT = 64;   // pack tile edge
+__host__ __device__ constexpr int pack_tiles_of(int n) { return (n - 1) / PT + 1; }   // n + 63 may not fit
 
 __device__ __forceinline__ int find_desc(const ca3dmm_pack_desc_t *d, int n, int tile)
 {
@@ -39,7 +40,7 @@ pack_kernel(const double *__restrict__ src_base, double *__restrict__ dst_base,
     for (int t = blockIdx.x; t < total_tiles; t += gridDim.x) {
         const ca3dmm_pack_desc_t d = descs[find_desc(descs, ndesc, t)];
         const int local = t - d.tile_begin;
-        const int tx = (d.rows + PT - 1) / PT;
+        const int tx = pack_tiles_of(d.rows);
         const int r0 = (local % tx) * PT, c0 = (local / tx) * PT;
         const double *src = reinterpret_cast<const double *>(
             reinterpret_cast<uintptr_t>(src_base) + (uintptr_t) d.src_off * sizeof(double));
@@ -224,7 +225,7 @@ extern "C" int ca3dmm_pack_tiles(ca3dmm_pack_desc_t *descs, int ndesc)
     for (int j = 0; j < ndesc; ++j) {
         descs[j].tile_begin = tiles;
         if (descs[j].rows > 0 && descs[j].cols > 0)
-            tiles += ((descs[j].rows + PT - 1) / PT) * ((descs[j].cols + PT - 1) / PT);
+            tiles += pack_tiles_of(descs[j].rows) * pack_tiles_of(descs[j].cols);
     }
     return tiles;
 }
@@ -307,21 +308,37 @@ copy_runs_kernel(const __grid_constant__ RunPieces<CAP> P, int npiece, int nch, 
     }
 }
 
+// Work items of a launch over these pieces, -1 when their number or the sizes leave
+// the kernel's 32-bit counts: it looks up to two chunks past a run's end.
+constexpr int RUN_MAX = 0x7fffffff - 4 * RUN_E;
+extern "C" long long ca3dmm_copy_runs_items(const ca3dmm_run_piece_t *pieces, int n)
+{
+    if (n < 0 || n > CA3DMM_MAX_RUN_PIECES) return -1;
+    long long groups = 0, nch = 0;
+    for (int i = 0; i < n; ++i) {
+        if (pieces[i].len <= 0 || pieces[i].runs <= 0) continue;
+        if (pieces[i].len > RUN_MAX || pieces[i].runs > RUN_MAX) return -1;
+        const long long g = (pieces[i].runs + RUN_GROUP - 1) / RUN_GROUP;
+        if (g > groups) groups = g;
+        if (run_chunks(pieces[i].len) > nch) nch = run_chunks(pieces[i].len);
+    }
+    const double items = (double) groups * n * (double) nch;
+    return items < 1e9 ? groups * n * nch : -1;
+}
+
 template <int CAP>
 static cudaError_t copy_runs_launch(const ca3dmm_run_piece_t *pieces, int n, cudaStream_t stream)
 {
     RunPieces<CAP> P;
     memset(&P, 0, sizeof(P));
-    long long groups = 0, nch = 0;
+    long long nch = 1;
     for (int i = 0; i < n; ++i) {
         P.p[i] = pieces[i];
-        const long long g = pieces[i].len > 0 ? (pieces[i].runs + RUN_GROUP - 1) / RUN_GROUP : 0;
-        if (g > groups) groups = g;
         if (run_chunks(pieces[i].len) > nch) nch = run_chunks(pieces[i].len);
     }
-    const long long items = groups * n * nch;
+    const long long items = ca3dmm_copy_runs_items(pieces, n);
     if (items == 0) return cudaSuccess;
-    if (items > 0x7fffffffLL - 1000000) return cudaErrorInvalidValue;
+    if (items < 0) return cudaErrorInvalidValue;
     const long long blocks = (items + 7) / 8, cap = (long long) ca3dmm_device_sm_count() * 64;
     copy_runs_kernel<CAP><<<(unsigned) (blocks < cap ? blocks : cap), 256, 0, stream>>>(
         P, n, (int) nch, (int) items);

@@ -178,13 +178,15 @@ int mat_redist_layouts_init(int nsrc, const int *src_rects, int nreq, const int 
             p->src = i; p->dst = j;
             p->srow = r0; p->scol = c0; p->nrow = r1 - r0; p->ncol = c1 - c0;
         }
-    double runs = 0, len = 0;     /* bound the launch's work items */
-    for (int k = 0; k < L->npiece; k++) {
-        if (L->pieces[k].nrow > runs) runs = L->pieces[k].nrow;
-        if (L->pieces[k].ncol > len) len = L->pieces[k].ncol;
+    if (L->npiece <= CA3DMM_MAX_RUN_PIECES) {
+        ca3dmm_run_piece_t rp[CA3DMM_MAX_RUN_PIECES];
+        memset(rp, 0, sizeof(rp));
+        for (int k = 0; k < L->npiece; k++) {
+            rp[k].len = L->pieces[k].ncol;
+            rp[k].runs = L->pieces[k].nrow;
+        }
+        L->by_value = ca3dmm_copy_runs_items(rp, L->npiece) >= 0;
     }
-    L->by_value = L->npiece <= CA3DMM_MAX_RUN_PIECES &&
-                  (runs / 4 + 1) * (len / 512 + 2) * L->npiece < 1e9;
     if (L->npiece > 0 && !L->by_value) {
         const size_t bytes = sizeof(ca3dmm_pack_desc_t) * (size_t) L->npiece;
         if (cudaMallocHost((void **) &L->desc_h, bytes) != cudaSuccess) L->desc_h = NULL;
