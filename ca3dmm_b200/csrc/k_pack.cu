@@ -256,7 +256,12 @@ copy_block_kernel(const double *__restrict__ src, long long lds, double *__restr
 // width), so a warp copies whole runs, two at a time with all their loads in
 // flight, four per item, up to RUN_E elements of them; its stores cover whole
 // lines.  Items go through the blocks in turn, four runs of each, so that the
-// blocks that share a destination row fill it at about the same time.
+// blocks that share a destination row fill it at about the same time -- as long as
+// the blocks are of about one size: each takes as many turns as the largest.  When
+// more than a quarter of the turns would be empty, the items follow the blocks one
+// after the other, each block with its own number (one 8000 x 8000 block beside 400
+// of 10 x 20, in turn 1657 us, tile copies 314, now 291; 60000 x 8000 beside 300 of
+// 1 x 20: 8690, 1357, now 1253).
 // 8000 x 8000 from 24 column strips to 4 x 6 blocks (116 pieces, 1.02 GB): 178 us,
 // 5.75 TB/s (one piece after the other 199-214; with default loads and stores in
 // place of the streaming ones, lines aligned, 373; 64 x 64 tiles from descriptors
@@ -265,23 +270,66 @@ copy_block_kernel(const double *__restrict__ src, long long lds, double *__restr
 constexpr int RUN_E = 512, RUN_GROUP = 4;
 __host__ __device__ inline int run_chunks(int len) { return (len + 15 + RUN_E - 1) / RUN_E; }
 
-template <int CAP>
-struct RunPieces {
-    ca3dmm_run_piece_t p[CAP];
+struct RunPiece {
+    const double *src;
+    double *dst;
+    int lds, ldd, len, runs;
+    int begin, nch;                                  // first item (blocks one after the other), chunks
 };
 
 template <int CAP>
+struct RunPieces {
+    RunPiece p[CAP];
+};
+
+struct RunItems {
+    int npiece, turn, total;                         // turn: chunks per block in turn (0: one after the other)
+};
+
+struct RunItem {
+    int piece, run0, run1, col0;                     // runs [run0, run1), from column col0 on
+};
+
+// Item -> what it copies; run0 == run1: nothing (an empty turn).
+__host__ __device__ inline RunItem run_item(const RunPiece *p, const RunItems &I, int item)
+{
+    RunItem o;
+    int g, c;
+    if (I.turn) {
+        const int ic = item / I.turn;
+        g = ic / I.npiece;
+        o.piece = ic - g * I.npiece;
+        c = item - ic * I.turn;
+    } else {
+        int lo = 0, hi = I.npiece - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (p[mid].begin <= item) lo = mid; else hi = mid - 1;
+        }
+        o.piece = lo;
+        g = (item - p[lo].begin) / p[lo].nch;
+        c = (item - p[lo].begin) - g * p[lo].nch;
+    }
+    const int runs = p[o.piece].runs;
+    o.col0 = c * RUN_E;
+    o.run0 = o.run1 = 0;
+    if (c < p[o.piece].nch && g < (runs + RUN_GROUP - 1) / RUN_GROUP) {
+        o.run0 = g * RUN_GROUP;
+        o.run1 = runs - o.run0 < RUN_GROUP ? runs : o.run0 + RUN_GROUP;
+    }
+    return o;
+}
+
+template <int CAP>
 __global__ void __launch_bounds__(256)
-copy_runs_kernel(const __grid_constant__ RunPieces<CAP> P, int npiece, int nch, int total_items)
+copy_runs_kernel(const __grid_constant__ RunPieces<CAP> P, const RunItems I)
 {
     const int lane = threadIdx.x & 31;
-    for (int item = blockIdx.x * 8 + (threadIdx.x >> 5); item < total_items; item += gridDim.x * 8) {
-        const int ic = item / nch, g = ic / npiece;
-        const ca3dmm_run_piece_t &d = P.p[ic - g * npiece];
-        const int c0 = (item - ic * nch) * RUN_E + lane;
-        const int r1 = min(d.runs, (g + 1) * RUN_GROUP);
-        if (g * RUN_GROUP >= d.runs || c0 - lane >= d.len + 15) continue;
-        for (int r = g * RUN_GROUP; r < r1; r += 2) {
+    for (int item = blockIdx.x * 8 + (threadIdx.x >> 5); item < I.total; item += gridDim.x * 8) {
+        const RunItem w = run_item(P.p, I, item);
+        const RunPiece &d = P.p[w.piece];
+        const int c0 = w.col0 + lane, r1 = w.run1;
+        for (int r = w.run0; r < r1; r += 2) {
             // each run's elements counted from the 128-byte line its destination starts
             // in, so that a warp's store covers whole lines
             const double *s0 = d.src + (long long) r * d.lds;
@@ -311,37 +359,66 @@ copy_runs_kernel(const __grid_constant__ RunPieces<CAP> P, int npiece, int nch, 
 // Work items of a launch over these pieces, -1 when their number or the sizes leave
 // the kernel's 32-bit counts: it looks up to two chunks past a run's end.
 constexpr int RUN_MAX = 0x7fffffff - 4 * RUN_E;
+static bool run_plan(const ca3dmm_run_piece_t *pieces, int n, RunPiece *p, RunItems &I)
+{
+    I = RunItems{0, 0, 0};
+    if (n < 0 || n > CA3DMM_MAX_RUN_PIECES) return false;
+    long long groups = 0, nch = 0, sum = 0;
+    for (int i = 0; i < n; ++i) {
+        const ca3dmm_run_piece_t &q = pieces[i];
+        if (q.len <= 0 || q.runs <= 0) continue;
+        if (q.len > RUN_MAX || q.runs > RUN_MAX) return false;
+        RunPiece &o = p[I.npiece++];
+        o.src = q.src; o.dst = q.dst;
+        o.lds = q.lds; o.ldd = q.ldd; o.len = q.len; o.runs = q.runs;
+        o.nch = run_chunks(q.len);
+        o.begin = (int) sum;
+        const long long g = (q.runs + RUN_GROUP - 1) / RUN_GROUP;
+        if (g > groups) groups = g;
+        if (o.nch > nch) nch = o.nch;
+        sum += g * o.nch;
+        if (sum > 1000000000) return false;
+    }
+    if (sum == 0) return true;
+    // (the groups and chunks of one block are at most sum: no overflow before the test)
+    const bool turn = (double) groups * I.npiece * (double) nch <= 1.25 * (double) sum;
+    I.turn = turn ? (int) nch : 0;
+    I.total = (int) (turn ? groups * I.npiece * nch : sum);
+    return true;
+}
+
 extern "C" long long ca3dmm_copy_runs_items(const ca3dmm_run_piece_t *pieces, int n)
 {
-    if (n < 0 || n > CA3DMM_MAX_RUN_PIECES) return -1;
-    long long groups = 0, nch = 0;
-    for (int i = 0; i < n; ++i) {
-        if (pieces[i].len <= 0 || pieces[i].runs <= 0) continue;
-        if (pieces[i].len > RUN_MAX || pieces[i].runs > RUN_MAX) return -1;
-        const long long g = (pieces[i].runs + RUN_GROUP - 1) / RUN_GROUP;
-        if (g > groups) groups = g;
-        if (run_chunks(pieces[i].len) > nch) nch = run_chunks(pieces[i].len);
-    }
-    const double items = (double) groups * n * (double) nch;
-    return items < 1e9 ? groups * n * nch : -1;
+    RunPieces<CA3DMM_MAX_RUN_PIECES> P;
+    RunItems I;
+    return run_plan(pieces, n, P.p, I) ? I.total : -1;
+}
+
+extern "C" int ca3dmm_copy_runs_item(const ca3dmm_run_piece_t *pieces, int n, int item, int *out5)
+{
+    RunPieces<CA3DMM_MAX_RUN_PIECES> P;
+    RunItems I;
+    if (!run_plan(pieces, n, P.p, I) || item < 0 || item >= I.total) return CA3DMM_EINVAL;
+    const RunItem w = run_item(P.p, I, item);
+    const RunPiece &d = P.p[w.piece];
+    // elements a lane may reach: the chunk, less the runs' offset in a line
+    out5[0] = w.piece;
+    out5[1] = w.run0;
+    out5[2] = w.run1;
+    out5[3] = w.col0;
+    out5[4] = d.len + 15 - w.col0 < RUN_E ? d.len + 15 : w.col0 + RUN_E;
+    return CA3DMM_OK;
 }
 
 template <int CAP>
 static cudaError_t copy_runs_launch(const ca3dmm_run_piece_t *pieces, int n, cudaStream_t stream)
 {
     RunPieces<CAP> P;
-    memset(&P, 0, sizeof(P));
-    long long nch = 1;
-    for (int i = 0; i < n; ++i) {
-        P.p[i] = pieces[i];
-        if (run_chunks(pieces[i].len) > nch) nch = run_chunks(pieces[i].len);
-    }
-    const long long items = ca3dmm_copy_runs_items(pieces, n);
-    if (items == 0) return cudaSuccess;
-    if (items < 0) return cudaErrorInvalidValue;
-    const long long blocks = (items + 7) / 8, cap = (long long) ca3dmm_device_sm_count() * 64;
-    copy_runs_kernel<CAP><<<(unsigned) (blocks < cap ? blocks : cap), 256, 0, stream>>>(
-        P, n, (int) nch, (int) items);
+    RunItems I;
+    if (!run_plan(pieces, n, P.p, I)) return cudaErrorInvalidValue;
+    if (I.total == 0) return cudaSuccess;
+    const long long blocks = (I.total + 7LL) / 8, cap = (long long) ca3dmm_device_sm_count() * 64;
+    copy_runs_kernel<CAP><<<(unsigned) (blocks < cap ? blocks : cap), 256, 0, stream>>>(P, I);
     ca3dmm_note_launch(1);
     return cudaGetLastError();
 }

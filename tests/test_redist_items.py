@@ -1,6 +1,7 @@
 """The numbering of the run copies' work items, checked on the CPU; runs that are
 almost as long as a 32-bit count, copied on the GPU."""
 import ctypes as C
+import random
 
 import pytest
 
@@ -14,15 +15,19 @@ class Piece(C.Structure):
         (n, C.c_int) for n in ("lds", "ldd", "len", "runs")]
 
 
-def items(shapes):
+def pieces(shapes):
     """shapes: [(len, runs)]"""
-    L = cb.lib()
-    L.ca3dmm_copy_runs_items.restype = C.c_longlong
     P = (Piece * max(1, len(shapes)))()
     for p, (length, runs) in zip(P, shapes):
         p.lds = p.ldd = p.len = length
         p.runs = runs
-    return L.ca3dmm_copy_runs_items(P, len(shapes))
+    return P
+
+
+def items(shapes):
+    L = cb.lib()
+    L.ca3dmm_copy_runs_items.restype = C.c_longlong
+    return L.ca3dmm_copy_runs_items(pieces(shapes), len(shapes))
 
 
 @pytest.mark.parametrize("length", [INT_MAX - 4096, INT_MAX - 2048, INT_MAX - 600, INT_MAX - 500,
@@ -36,6 +41,76 @@ def test_counts_near_the_limit(length, turn):
 
 def test_no_items_of_empty_pieces():
     assert items([]) == 0 and items([(0, 5), (5, 0)]) == 0
+
+
+def layouts():
+    rng = random.Random(5)
+    out = [[(1, 1)], [(333, 7)] * 24, [(20, 1600), (33, 3), (512, 1), (1, 1)],
+           [(8000, 8000)] + [(20, 10)] * 400, [(8, 3900)] + [(8, 1)] * 511,
+           [(334, 7981)] * 24 + [(334, 1)] * 456, [(40000, 3), (0, 4), (4, 0), (17, 90)]]
+    for _ in range(30):
+        n = rng.choice([1, 2, 63, 64, 65, 200, 512])
+        top = rng.choice([4, 40, 400, 4000])
+        out.append([(rng.randint(0, top), rng.randint(0, max(1, 3000 // top))) for _ in range(n)])
+    return out
+
+
+@pytest.mark.parametrize("shapes", layouts(), ids=lambda s: "%dx" % len(s))
+def test_items_cover_every_run_once(shapes):
+    """Every column of every run, wherever in a line it starts, in one item; at most a
+    fifth of the items are empty turns."""
+    L = cb.lib()
+    P, n, out = pieces(shapes), items(shapes), (C.c_int * 5)()
+    full = [s for s in shapes if s[0] > 0 and s[1] > 0]
+    seen = [{} for _ in full]
+    empty = 0
+    for i in range(n):
+        assert L.ca3dmm_copy_runs_item(P, len(shapes), i, out) == 0
+        k, r0, r1, c0, c1 = out
+        if r0 == r1:
+            empty += 1
+            continue
+        assert 0 <= r0 < r1 <= full[k][1] and 0 <= c0 < c1
+        seen[k].setdefault((r0, r1), []).append((c0, c1))
+    for (length, runs), got in zip(full, seen):
+        spans = sorted(got)
+        assert [a for a, _ in spans] == [0] + [b for _, b in spans[:-1]] and spans[-1][1] == runs
+        for chunks in got.values():
+            chunks.sort()
+            assert chunks[0][0] == 0 and all(a[1] == b[0] for a, b in zip(chunks, chunks[1:]))
+            assert chunks[-1][1] == length + 15
+    assert empty <= 0.2 * n
+    assert L.ca3dmm_copy_runs_item(P, len(shapes), n, out) != 0
+
+
+def rects(heights, widths, r0=0):
+    out = []
+    for h in heights:
+        c0 = 0
+        for w in widths:
+            out.append((r0, c0, h, w))
+            c0 += w
+        r0 += h
+    return out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("src,dst", [
+    (rects([3001], [77, 400, 5, 900]), rects([2990] + [1] * 11, [1382])),
+    (rects([60], [8000]), rects([10], [20] * 400) + rects([50], [8000], 10)),
+    (rects([5000], [8]), rects([1] * 20 + [4900] + [1] * 80, [8])),
+    (rects([700], [33, 64, 20, 31, 127, 129, 240, 3]), rects([1, 699], [300, 347])),
+])
+def test_uneven_layouts(cuda, src, dst):
+    import torch
+    rows, cols = max(r + h for r, _, h, _ in src), max(c + w for _, c, _, w in src)
+    G = torch.rand(rows, cols, dtype=torch.float64, device="cuda")
+    cut = lambda R: [G[r:r + h, c:c + w].contiguous() for r, c, h, w in R]
+    S, want = cut(src), cut(dst)
+    D = [torch.full_like(w, -7.0) for w in want]
+    lay = cb.RedistLayouts(src, dst)
+    assert lay.ok and lay.exec(S, [x.shape[1] for x in S], D, [x.shape[1] for x in D]) == 0
+    assert all(torch.equal(a, b) for a, b in zip(D, want))
 
 
 @pytest.mark.gpu
