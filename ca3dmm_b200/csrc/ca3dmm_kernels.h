@@ -154,7 +154,7 @@ typedef struct {
 long long ca3dmm_copy_runs_items(const ca3dmm_run_piece_t *pieces, int n);   /* -1: not one launch */
 /* What a work item copies: non-empty piece, runs [1], [2), columns [3], [4) (both counted from
  * the 128-byte line that each destination run starts in). */
-int ca3dmm_copy_runs_item(const ca3dmm_run_piece_t *pieces, int n, int item, int *out5);
+int ca3dmm_copy_runs_item(const ca3dmm_run_piece_t *pieces, int n, long long item, int *out5);
 int ca3dmm_copy_runs_launch(const ca3dmm_run_piece_t *pieces, int n, cudaStream_t stream);
 
 /* One column-major block copy dst[r + c*ldd] = src[r + c*lds] (rows x cols),

@@ -267,14 +267,31 @@ copy_block_kernel(const double *__restrict__ src, long long lds, double *__restr
 // place of the streaming ones, lines aligned, 373; 64 x 64 tiles from descriptors
 // in memory 206).  The call: 242 -> 206 us, with the upload of the descriptors and
 // the wait before it gone.
-constexpr int RUN_E = 512, RUN_GROUP = 4;
-__host__ __device__ inline int run_chunks(int len) { return (len + 15 + RUN_E - 1) / RUN_E; }
+// Runs of up to RUN_NARROW elements are too short for that: two of them in flight are
+// less than the memory's latency asks for.  An item takes as many as fill 64 loads of
+// every lane, half of them in flight; runs of up to 16 elements lie side by side in
+// a warp.  Into 8 row blocks (256 MB each way): 1600000 x 20 in 106 us (385 two runs
+// at a time, 167 by tile copies), 1000000 x 32 106 (263, 128), 500000 x 64 105 (164,
+// 110), 250000 x 128 106 (119, 109); 400 strips of 20, 64, 100 columns to one block
+// 219, 390, 528 us (500, 560, 650; 324, 438, 680).  At 160 and 200 columns both take
+// the same time, at 256 whole runs 104 us and this 107; with 16 loads in flight in
+// twice the warps 1 to 2 % more, with loads that L1 keeps up to 10 %.
+constexpr int RUN_E = 512, RUN_GROUP = 4, RUN_NARROW = 128, RUN_LOADS = 32;
+__host__ __device__ inline bool run_narrow(int len) { return len <= RUN_NARROW; }
+// narrow: loads per run, and log2 of the lanes that share one
+__host__ __device__ inline int run_loads(int len) { return len <= 32 ? 1 : len <= 64 ? 2 : 4; }
+__host__ __device__ inline int run_lanes(int len) { return len > 16 ? 5 : len > 8 ? 4 : len > 4 ? 3 : len > 2 ? 2 : len > 1 ? 1 : 0; }
+inline int run_chunks(int len) { return run_narrow(len) ? 1 : (len + 15 + RUN_E - 1) / RUN_E; }
+inline int run_group(int len)
+{
+    return run_narrow(len) ? 2 * (RUN_LOADS / run_loads(len)) << (5 - run_lanes(len)) : RUN_GROUP;
+}
 
 struct RunPiece {
     const double *src;
     double *dst;
     int lds, ldd, len, runs;
-    int begin, nch;                                  // first item (blocks one after the other), chunks
+    int begin, nch, group;               // first item (blocks one after the other), chunks, runs per item
 };
 
 template <int CAP>
@@ -310,14 +327,47 @@ __host__ __device__ inline RunItem run_item(const RunPiece *p, const RunItems &I
         g = (item - p[lo].begin) / p[lo].nch;
         c = (item - p[lo].begin) - g * p[lo].nch;
     }
-    const int runs = p[o.piece].runs;
+    const int runs = p[o.piece].runs, group = p[o.piece].group;
     o.col0 = c * RUN_E;
     o.run0 = o.run1 = 0;
-    if (c < p[o.piece].nch && g < (runs + RUN_GROUP - 1) / RUN_GROUP) {
-        o.run0 = g * RUN_GROUP;
-        o.run1 = runs - o.run0 < RUN_GROUP ? runs : o.run0 + RUN_GROUP;
+    if (c < p[o.piece].nch && (long long) g * group < runs) {
+        o.run0 = g * group;
+        o.run1 = runs - o.run0 < group ? runs : o.run0 + group;
     }
     return o;
+}
+
+// An item of narrow runs, U loads each.
+template <int U>
+__device__ __forceinline__ void copy_narrow(const RunPiece &d, int run0, int run1, int lane)
+{
+    const int lg = U == 1 ? run_lanes(d.len) : 5, sub = 32 >> lg;
+    const int col = lane & ((1 << lg) - 1);
+    const long long ds = (long long) sub * d.lds, dd = (long long) sub * d.ldd;
+    const long long first = run0 + (lane >> lg);
+    const double *s = d.src + first * d.lds + col;
+    double *t = d.dst + first * d.ldd + col;
+    int left = (run1 - (int) first + sub - 1) >> (5 - lg);      // runs of this lane
+#pragma unroll 1
+    for (; left > 0; left -= RUN_LOADS / U) {
+        double v[RUN_LOADS];
+#pragma unroll
+        for (int i = 0; i < RUN_LOADS / U; ++i) {
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                v[i * U + u] = i < left && col + 32 * u < d.len ? __ldcs(s + 32 * u) : 0.0;
+            s += ds;
+            asm volatile("" : "+l"(s));              // one address at a time
+        }
+#pragma unroll
+        for (int i = 0; i < RUN_LOADS / U; ++i) {
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (i < left && col + 32 * u < d.len) __stcs(t + 32 * u, v[i * U + u]);
+            t += dd;
+            asm volatile("" : "+l"(t));
+        }
+    }
 }
 
 template <int CAP>
@@ -356,24 +406,42 @@ copy_runs_kernel(const __grid_constant__ RunPieces<CAP> P, const RunItems I)
     }
 }
 
+// The same for blocks of narrow runs: a kernel of its own, whose warps need half the
+// registers.
+template <int CAP>
+__global__ void __launch_bounds__(256, 2)
+copy_narrow_runs_kernel(const __grid_constant__ RunPieces<CAP> P, const RunItems I)
+{
+    const int lane = threadIdx.x & 31;
+    for (int item = blockIdx.x * 8 + (threadIdx.x >> 5); item < I.total; item += gridDim.x * 8) {
+        const RunItem w = run_item(P.p, I, item);
+        const RunPiece &d = P.p[w.piece];
+        const int loads = run_loads(d.len);
+        if (loads == 1) copy_narrow<1>(d, w.run0, w.run1, lane);
+        else if (loads == 2) copy_narrow<2>(d, w.run0, w.run1, lane);
+        else copy_narrow<4>(d, w.run0, w.run1, lane);
+    }
+}
+
 // Work items of a launch over these pieces, -1 when their number or the sizes leave
 // the kernel's 32-bit counts: it looks up to two chunks past a run's end.
 constexpr int RUN_MAX = 0x7fffffff - 4 * RUN_E;
-static bool run_plan(const ca3dmm_run_piece_t *pieces, int n, RunPiece *p, RunItems &I)
+static bool run_plan(const ca3dmm_run_piece_t *pieces, int n, bool narrow, RunPiece *p, RunItems &I)
 {
     I = RunItems{0, 0, 0};
     if (n < 0 || n > CA3DMM_MAX_RUN_PIECES) return false;
     long long groups = 0, nch = 0, sum = 0;
     for (int i = 0; i < n; ++i) {
         const ca3dmm_run_piece_t &q = pieces[i];
-        if (q.len <= 0 || q.runs <= 0) continue;
+        if (q.len <= 0 || q.runs <= 0 || run_narrow(q.len) != narrow) continue;
         if (q.len > RUN_MAX || q.runs > RUN_MAX) return false;
         RunPiece &o = p[I.npiece++];
         o.src = q.src; o.dst = q.dst;
         o.lds = q.lds; o.ldd = q.ldd; o.len = q.len; o.runs = q.runs;
         o.nch = run_chunks(q.len);
+        o.group = run_group(q.len);
         o.begin = (int) sum;
-        const long long g = (q.runs + RUN_GROUP - 1) / RUN_GROUP;
+        const long long g = (q.runs - 1LL) / o.group + 1;
         if (g > groups) groups = g;
         if (o.nch > nch) nch = o.nch;
         sum += g * o.nch;
@@ -390,19 +458,28 @@ static bool run_plan(const ca3dmm_run_piece_t *pieces, int n, RunPiece *p, RunIt
 extern "C" long long ca3dmm_copy_runs_items(const ca3dmm_run_piece_t *pieces, int n)
 {
     RunPieces<CA3DMM_MAX_RUN_PIECES> P;
-    RunItems I;
-    return run_plan(pieces, n, P.p, I) ? I.total : -1;
+    RunItems wide, narrow;
+    return run_plan(pieces, n, false, P.p, wide) && run_plan(pieces, n, true, P.p, narrow)
+               ? (long long) wide.total + narrow.total : -1;
 }
 
-extern "C" int ca3dmm_copy_runs_item(const ca3dmm_run_piece_t *pieces, int n, int item, int *out5)
+extern "C" int ca3dmm_copy_runs_item(const ca3dmm_run_piece_t *pieces, int n, long long item, int *out5)
 {
     RunPieces<CA3DMM_MAX_RUN_PIECES> P;
     RunItems I;
-    if (!run_plan(pieces, n, P.p, I) || item < 0 || item >= I.total) return CA3DMM_EINVAL;
-    const RunItem w = run_item(P.p, I, item);
+    if (item < 0 || !run_plan(pieces, n, false, P.p, I)) return CA3DMM_EINVAL;
+    const bool narrow = item >= I.total;
+    if (narrow) item -= I.total;
+    if (!run_plan(pieces, n, narrow, P.p, I) || item >= I.total) return CA3DMM_EINVAL;
+    const RunItem w = run_item(P.p, I, (int) item);
     const RunPiece &d = P.p[w.piece];
-    // elements a lane may reach: the chunk, less the runs' offset in a line
-    out5[0] = w.piece;
+    out5[0] = 0;
+    for (int i = 0, of = 0; of < w.piece || run_narrow(pieces[i].len) != narrow || pieces[i].len <= 0 ||
+                            pieces[i].runs <= 0; ++i) {
+        if (pieces[i].len <= 0 || pieces[i].runs <= 0) continue;
+        ++out5[0];
+        if (run_narrow(pieces[i].len) == narrow) ++of;
+    }
     out5[1] = w.run0;
     out5[2] = w.run1;
     out5[3] = w.col0;
@@ -415,11 +492,16 @@ static cudaError_t copy_runs_launch(const ca3dmm_run_piece_t *pieces, int n, cud
 {
     RunPieces<CAP> P;
     RunItems I;
-    if (!run_plan(pieces, n, P.p, I)) return cudaErrorInvalidValue;
-    if (I.total == 0) return cudaSuccess;
-    const long long blocks = (I.total + 7LL) / 8, cap = (long long) ca3dmm_device_sm_count() * 64;
-    copy_runs_kernel<CAP><<<(unsigned) (blocks < cap ? blocks : cap), 256, 0, stream>>>(P, I);
-    ca3dmm_note_launch(1);
+    const long long cap = (long long) ca3dmm_device_sm_count() * 64;
+    for (int narrow = 0; narrow < 2; ++narrow) {
+        if (!run_plan(pieces, n, narrow, P.p, I)) return cudaErrorInvalidValue;
+        if (I.total == 0) continue;
+        const long long blocks = (I.total + 7LL) / 8;
+        const unsigned grid = (unsigned) (blocks < cap ? blocks : cap);
+        if (narrow) copy_narrow_runs_kernel<CAP><<<grid, 256, 0, stream>>>(P, I);
+        else copy_runs_kernel<CAP><<<grid, 256, 0, stream>>>(P, I);
+        ca3dmm_note_launch(1);
+    }
     return cudaGetLastError();
 }
 
