@@ -85,9 +85,10 @@ int ca3dmm_dgemm_launch_ranges_tn(const void *dev_plan, int nprob,
  * tile order (tn counts tile_n columns), the CTAs' lists of them and the
  * number of counters (cut tiles, one zeroed int each; the launch leaves them
  * zero); segs and order hold ca3dmm_dgemm_segments_max entries, cta_begin 149.
- * CA3DMM_EINVAL when the product has too many tiles for this form (max 0). */
+ * CA3DMM_EINVAL when such a product goes to the grouped kernel (max 0). */
 #define CA3DMM_DGEMM_CHUNK 16        /* 16-k blocks per accumulation chain */
 #define CA3DMM_DGEMM_SEG_CTAS 148
+#define CA3DMM_DGEMM_SEG_TILES (16 * CA3DMM_DGEMM_SEG_CTAS)   /* of a product that may be cut */
 typedef struct {
     int tm, tn;          /* tile */
     int kt0, kt1;        /* 16-k blocks [kt0, kt1) */

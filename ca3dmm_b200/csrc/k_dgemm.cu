@@ -404,13 +404,18 @@ dgemm_dmma_grouped(const CUtensorMap *__restrict__ tmaps, const DProb *__restric
 // that counts last adds the partials in segment order and stores C.  No CTA
 // ever waits for another, and the order of the sum is fixed.
 //
-// Inside a segment the accumulators restart every `chunk` k tiles: the partial
+// Inside a segment the accumulators restart after at most CHUNK k tiles: the partial
 // sums move to a running total in TMEM, which this kernel's MMAs leave free
 // (the same thread writes and reads its words, 128 per thread at 128 columns).
 // Rounding errors grow with the length of a chain of additions, so chunks of
 // 256 k keep the result at least as accurate as the k sub-slabs of up to
 // several thousand k, summed by a kernel of their own, that these shapes ran as
-// before.  (All warps at once lost 1.2 us per chunk of 35 us.)
+// before; a segment of more takes one chain more than it must, all of one length.
+// All warps restart at the same block: the additions use the pipe of the
+// MMAs, 1.3 us per chunk of 35 us (0.2 of it the moves to and from TMEM).  With the
+// warps of rows 64 .. 127 half a chunk later they lost 1.8 us, with one m16 tile of
+// a warp at a time, spread over the chunk, 5: an addition waits for the MMAs of the
+// other warp (4736 x 1024 x 8192: 2364, 2427, 2674 us; without restarts 2277, as it is 2345).
 __device__ __forceinline__ void tmem_ld32_wait(uint32_t taddr, uint32_t (&v)[32])
 {
     asm volatile(
@@ -483,7 +488,8 @@ __global__ void __launch_bounds__(THREADS, 1)
 dgemm_dmma_segments(const __grid_constant__ CUtensorMap map_a,
                     const __grid_constant__ CUtensorMap map_b, const __grid_constant__ DProb prob,
                     const __grid_constant__ SegOrder order,
-                    const ca3dmm_dgemm_seg_t *__restrict__ segs, int chunk, double2 *__restrict__ partials, int *__restrict__ counters, int *status,
+                    const ca3dmm_dgemm_seg_t *__restrict__ segs, int split,
+                    double2 *__restrict__ partials, int *__restrict__ counters, int *status,
                     unsigned long long limit_ns)
 {
     extern __shared__ uint8_t smem_raw[];
@@ -586,9 +592,8 @@ dgemm_dmma_segments(const __grid_constant__ CUtensorMap map_a,
     for (int pos = first; pos < end && ok; pos += step) {
         const ca3dmm_dgemm_seg_t &sg = segs[pos];
         int left = sg.kt1 - sg.kt0;
-        // the warps of rows 64 .. 127 start with half a chunk: of an SM quarter's two
-        // warps one keeps the tensor pipe busy while the other moves its sums
-        int len = warp >= CONSUMER_WARPS / 2 && left > chunk ? chunk / 2 : chunk;
+        const int chains = (left + CA3DMM_DGEMM_CHUNK - 1) / CA3DMM_DGEMM_CHUNK + (left >= split);
+        const int chunk = (left + chains - 1) / chains;
         bool totalled = false;
         for (;;) {
 #pragma unroll
@@ -597,8 +602,7 @@ dgemm_dmma_segments(const __grid_constant__ CUtensorMap map_a,
                 for (int j = 0; j < 4; ++j)
 #pragma unroll
                     for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.0;
-            const int now = min(left, len);
-            len = chunk;
+            const int now = min(left, chunk);
             ok = k_loop<AK, TBN>(smem, full, empty, now, it, acc, &abort_flag, status, limit_ns,
                                  producer, issue_one, wm, wn, g, t, lane);
             if (!ok) break;
@@ -939,13 +943,19 @@ extern "C" int ca3dmm_dgemm_launch_ranges_tn(const void *dev_plan, int nprob,
 // their number / grid.  The cuts depend on (m, n, k) alone, not on the tile
 // width, the raster or the operands' layout, and neither do the results.
 //
-// When (all in units of a 16-k block of one tile, 2.25 us of an SM): whole
-// tiles take ceil(T / 148) K.  Segments take T K / 148 and, for finishing cut
-// tiles, about 1.1 (writing a partial, the counter) and 0.4 per partial read
-// back.  At 1000^3 (T = 64, K = 63) that is 63 against 31: measured 148 us
-// against 70; at 2048^3 the sub-slabs of 512 k and their sum took 574 us, the
-// segments 523 (2.3 us per block of the 93 % busy tensor pipe, 3 us to start, 3
-// for the cut tiles).
+// When (all in units of a 16-k block of one tile, 2.2 us of an SM): whole tiles
+// take ceil(T / 148) K.  Cut tiles take T K / grid and, for writing the partials
+// and adding them up, from 2 (CTAs inside one tile each) to 7 (every CTA between two
+// tiles): fitted to 530 shapes of 1 to 2368 tiles and 2 to 1024 blocks, where the
+// choice is within 7 % of the better one and 0.06 % on average (with 1.9 in place of
+// 2 to 7 it lost up to 16 %, 1408 x 1408 x 256 took 78 us and now takes 68).  At 1000^3
+// (T = 64, K = 63) 31 blocks against 63: measured 70 us against 148.
+// Products of four rounds or more that equal shares would not shorten by 2 % stay
+// with the grouped kernel (one chain over k, no restarts).  Whole tiles run here
+// with restarts, those of up to one chunk in two chains, as a cut tile has on
+// average: the errors do not grow where the tiles are left whole (1408 x 1408 x 256
+// in one chain 1.86e-16 of |A||B| rms, cut 1.46e-16, in two 1.27e-16; without the
+// restarts long products are 3 to 5 % faster and their errors twice as large).
 // A product of few blocks is not spread over all SMs: the partials read back by
 // the last CTA of a tile grow with the parts, so the number of CTAs is at most
 // sqrt(2.5 T T K).  From k = 512 on a share is at least one chunk: chains of 256 k
@@ -955,12 +965,13 @@ extern "C" int ca3dmm_dgemm_launch_ranges_tn(const void *dev_plan, int nprob,
 // seven INT8 slices that are to match it, 4.5e-16).  The price at 768^3: 16 blocks
 // per CTA instead of 12.
 namespace {
-constexpr int SEG_SMS = 148, SEG_MAX_TILES = 16 * SEG_SMS, SEG_RASTER = 8;
+constexpr int SEG_SMS = CA3DMM_DGEMM_SEG_CTAS, SEG_RASTER = 8;
 
 struct SegShape {
     long long T, K;              // 128 x 128 tiles, 16-k blocks of a tile
     int tiles_m, tiles_n, grid;
     long long whole;             // rounds of whole tiles before the cut ones (-1: nothing is cut)
+    int split;                   // segments of at least so many blocks take one chain more
 };
 
 bool seg_shape(int m, int n, int k, SegShape &s)
@@ -970,7 +981,8 @@ bool seg_shape(int m, int n, int k, SegShape &s)
     s.tiles_n = (n + 127) / 128;
     s.T = (long long) s.tiles_m * s.tiles_n;
     s.K = ((long long) k + BK - 1) / BK;
-    if (s.T > SEG_MAX_TILES) return false;
+    s.split = CA3DMM_DGEMM_CHUNK + 1;
+    if (s.T > CA3DMM_DGEMM_SEG_TILES) return false;
     const double dp = (double) ((s.T + SEG_SMS - 1) / SEG_SMS) * (double) s.K;
     double g = std::sqrt(2.5 * (double) s.T * (double) s.T * (double) s.K);
     if (g > SEG_SMS) g = SEG_SMS;
@@ -978,13 +990,15 @@ bool seg_shape(int m, int n, int k, SegShape &s)
     if (s.K >= 2 * CA3DMM_DGEMM_CHUNK && g > (double) (s.T * s.K / CA3DMM_DGEMM_CHUNK))
         g = (double) (s.T * s.K / CA3DMM_DGEMM_CHUNK);
     s.grid = g < 1.0 ? 1 : (int) g;
-    const double parts = s.T >= s.grid ? 2.0 : (double) s.grid / (double) s.T + 1.0;
-    const double seg = (double) s.T * (double) s.K / s.grid + 1.1 + 0.4 * parts;
-    if (seg < 0.98 * dp) {
+    const double share = (double) s.T * (double) s.K / s.grid;
+    if (s.T >= 4 * SEG_SMS && share + 1.9 >= 0.98 * dp) return false;
+    const double spread = s.T < s.grid ? (double) s.T / s.grid : 1.0;
+    if (share + 2.0 + 5.0 * spread < dp) {
         s.whole = s.T / s.grid > 1 ? s.T / s.grid - 1 : 0;
     } else {
         s.whole = -1;
         s.grid = s.T < SEG_SMS ? (int) s.T : SEG_SMS;
+        s.split = 6;
     }
     return true;
 }
@@ -1003,8 +1017,6 @@ extern "C" int ca3dmm_dgemm_segments_max(int m, int n, int k)
 {
     SegShape s;
     if (!seg_shape(m, n, k, s)) return 0;
-    // several rounds that cutting would not shorten: whole tiles in raster order
-    if (s.whole < 0 && s.T >= 4 * SEG_SMS) return 0;
     return (int) (2 * (s.T + s.grid));
 }
 
@@ -1104,8 +1116,9 @@ extern "C" int ca3dmm_dgemm_segments(int m, int n, int k, int tile_n, ca3dmm_dge
 namespace {
 template <bool AK, int TBN>
 cudaError_t seg_launch_one(int grid, const CUtensorMap *tm, const DProb &prob, const SegOrder &o,
-                           const ca3dmm_dgemm_seg_t *segs, double2 *partials, int *counters,
-                           int *status, unsigned long long limit, cudaStream_t stream)
+                           const ca3dmm_dgemm_seg_t *segs, int split, double2 *partials,
+                           int *counters, int *status, unsigned long long limit,
+                           cudaStream_t stream)
 {
     static std::atomic<unsigned long long> done{0};      // as dgemm_attr_once
     int dev = 0;
@@ -1120,7 +1133,7 @@ cudaError_t seg_launch_one(int grid, const CUtensorMap *tm, const DProb &prob, c
         done.fetch_or(bit, std::memory_order_release);
     }
     dgemm_dmma_segments<AK, TBN><<<grid, THREADS, DTile<TBN>::SMEM_BYTES, stream>>>(
-        tm[0], tm[1], prob, o, segs, CA3DMM_DGEMM_CHUNK, partials, counters, status, limit);
+        tm[0], tm[1], prob, o, segs, split, partials, counters, status, limit);
     return cudaGetLastError();
 }
 }  // namespace
@@ -1148,18 +1161,20 @@ extern "C" int ca3dmm_dgemm_launch_segments(const void *host_plan, int nprob,
         grid = ca3dmm_device_sm_count();
         if (grid > hi - lo) grid = hi - lo;
     }
+    SegShape s;
+    if (!seg_shape(prob.m, prob.n, prob.k, s)) return CA3DMM_EINVAL;
     const unsigned long long limit = (unsigned long long) (timeout_s * 1e9);
     double2 *ws = static_cast<double2 *>(partials);
     cudaError_t err;
     if (tile_n == 128)
-        err = a_kmajor ? seg_launch_one<true, 128>(grid, tm, prob, o, dev_segs, ws, counters,
+        err = a_kmajor ? seg_launch_one<true, 128>(grid, tm, prob, o, dev_segs, s.split, ws, counters,
                                                     dev_status, limit, stream)
-                       : seg_launch_one<false, 128>(grid, tm, prob, o, dev_segs, ws, counters,
+                       : seg_launch_one<false, 128>(grid, tm, prob, o, dev_segs, s.split, ws, counters,
                                                      dev_status, limit, stream);
     else
-        err = a_kmajor ? seg_launch_one<true, 64>(grid, tm, prob, o, dev_segs, ws, counters,
+        err = a_kmajor ? seg_launch_one<true, 64>(grid, tm, prob, o, dev_segs, s.split, ws, counters,
                                                    dev_status, limit, stream)
-                       : seg_launch_one<false, 64>(grid, tm, prob, o, dev_segs, ws, counters,
+                       : seg_launch_one<false, 64>(grid, tm, prob, o, dev_segs, s.split, ws, counters,
                                                     dev_status, limit, stream);
     CA3DMM_CUDA_TRY(err);
     ca3dmm_note_launch(1);
