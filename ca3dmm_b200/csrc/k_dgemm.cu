@@ -1003,6 +1003,28 @@ bool seg_shape(int m, int n, int k, SegShape &s)
     return true;
 }
 
+// Cut points of the tiles after the whole ones, in blocks; one within 1/16 of a
+// share (or one block) of a tile's edge moves there, which saves a partial.
+// Returns the number of whole tiles.
+long long seg_cuts(const SegShape &s, long long (&cut)[SEG_SMS + 1])
+{
+    const int G = s.grid;
+    const long long dp = s.whole < 0 ? s.T : s.whole * G;
+    const long long U = (s.T - dp) * s.K;
+    const long long slack = U / G / 16 > 1 ? U / G / 16 : 1;
+    for (int c = 0; c <= G; ++c) {
+        long long u = U > 0 ? U * c / G : 0;
+        if (c > 0 && c < G) {
+            const long long r = u % s.K;
+            if (r <= slack && r < s.K - r) u -= r;
+            else if (s.K - r <= slack) u += s.K - r;
+            if (u < cut[c - 1]) u = cut[c - 1];
+        }
+        cut[c] = u;
+    }
+    return dp;
+}
+
 void seg_tile(const SegShape &s, long long tile, int &tm, int &tn)
 {
     const long long per = (long long) SEG_RASTER * s.tiles_n, b = tile / per, r = tile % per;
@@ -1024,8 +1046,16 @@ extern "C" size_t ca3dmm_dgemm_segments_ws_bytes(int m, int n, int k)
 {
     SegShape s;
     if (!seg_shape(m, n, k, s) || s.whole < 0) return 0;
-    // every cut adds one partial to the tile it falls into, whose first it also makes
-    return (size_t) 2 * (size_t) s.grid * BM * 128 * sizeof(double);
+    // every cut inside a tile adds a partial, the first of a tile's two
+    long long cut[SEG_SMS + 1], tile = -1, last = 0, slots = 0;
+    seg_cuts(s, cut);
+    for (int c = 1; c < s.grid; ++c) {
+        if (cut[c] % s.K == 0 || cut[c] == last) continue;
+        last = cut[c];
+        slots += last / s.K == tile ? 1 : 2;
+        tile = last / s.K;
+    }
+    return (size_t) slots * BM * 128 * sizeof(double);
 }
 
 extern "C" int ca3dmm_dgemm_segments(int m, int n, int k, int tile_n, ca3dmm_dgemm_seg_t *segs,
@@ -1036,23 +1066,9 @@ extern "C" int ca3dmm_dgemm_segments(int m, int n, int k, int tile_n, ca3dmm_dge
     *nseg = *grid = *ncounter = 0;
     if (!seg_shape(m, n, k, s) || (tile_n != 128 && tile_n != 64)) return CA3DMM_EINVAL;
     const int G = s.grid;
-    const long long dp = s.whole < 0 ? s.T : s.whole * G;       // whole tiles
-    const long long U = (s.T - dp) * s.K;                       // blocks of the others
-    // cut points in blocks; one within 1/16 of a share (or one block) of a tile's
-    // edge moves there, which saves a partial
-    const long long slack = U / G / 16 > 1 ? U / G / 16 : 1;
     int ns = 0, nc = 0, slots = 0;
     long long cut[SEG_SMS + 1];
-    for (int c = 0; c <= G; ++c) {
-        long long u = U > 0 ? U * c / G : 0;
-        if (c > 0 && c < G) {
-            const long long r = u % s.K;
-            if (r <= slack && r < s.K - r) u -= r;
-            else if (s.K - r <= slack) u += s.K - r;
-            if (u < cut[c - 1]) u = cut[c - 1];
-        }
-        cut[c] = u;
-    }
+    const long long dp = seg_cuts(s, cut);                      // whole tiles
     // segments in tile order, each with the CTA that runs it
     int *who = static_cast<int *>(malloc(sizeof(int) * (size_t) (2 * (s.T + G) + 1)));
     if (!who) return CA3DMM_ENOMEM;
