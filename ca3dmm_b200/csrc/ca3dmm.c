@@ -1349,7 +1349,7 @@ static int launch_guard_check(const ca3dmm_engine_p e, const plan_t *pl, int *st
  * tile rows each) run as one GEMM launch per band on `st`, and the
  * reconstruction of band b runs on the auxiliary stream as soon as band b's
  * residue planes are complete -- beside the GEMM of band b + 1 (two blocks per
- * SM fit next to the GEMM's CTA: 2 x 256 x 48 registers and 2 x 4 KB of shared
+ * SM fit next to the GEMM's CTA: 384 x 80 + 2 x 256 x 64 registers, no shared
  * memory, with the same shared-memory carveout).  Returns the number of bands
  * so run (0: not overlapped). */
 static int crt_overlapped_gemm(ca3dmm_engine_p e, plan_t *pl, int *status_d, cudaStream_t st,

@@ -62,6 +62,7 @@ struct CrtTile {
     static constexpr size_t kSmem = (size_t) kStages * kStageBytes + (2 * kStages + 4) * 8 + 1024;
 };
 constexpr int C_THREADS = 384;                   // 12 warps
+constexpr int C_BLOCKS = 2;                      // its registers: half an SM's (shared memory holds one)
 constexpr int C_ISSUERS = 2;
 constexpr int C_EPI_WARPS = 8;
 constexpr int GROUP_CACHE = 512;
@@ -417,7 +418,7 @@ struct alignas(16) CrtItem {
 constexpr int ITEM_READERS = 1 + C_ISSUERS + C_EPI_WARPS;
 
 template <int TN>
-__global__ void __launch_bounds__(C_THREADS, 2)
+__global__ void __launch_bounds__(C_THREADS, C_BLOCKS)
 crt_gemm_kernel(const CrtGroup *__restrict__ groups, int ngroup, int nmod,
                 const ca3dmm_tile_ranges_t rg, int total_items,
                 unsigned char *__restrict__ work, int *status, unsigned long long limit_ns)
@@ -764,7 +765,7 @@ __host__ __device__ constexpr Recon<N> make_recon()
 // modulo 2^128, which holds it exactly in two's complement because |C'| <= k
 // 2^(2P) <= 2^123.  The weights are compile-time constants.
 // What bounds it is instruction issue (about 130 per entry, half of the issue slots
-// of the 32 warps its 64 registers allow at 15 moduli), then the residues' loads:
+// of the 32 warps its 64 registers allow), then the residues' loads:
 // 8000 x 8000 entries of 15 moduli in 490 us (two bands), 1.47 GB at 3 TB/s, 4.2 M
 // entries in 33 us, 240 M of a batch in 1.60 ms.  With one limb product per modulus
 // and limb, the value rounded through a 64-bit window, and each lane storing its own
@@ -774,7 +775,17 @@ __host__ __device__ constexpr Recon<N> make_recon()
 // rows [r0, r1) of group g0; several: every row of groups [g0, g1), numbered by
 // the groups' rc_begin prefix (found by a search over a shared copy), so that the
 // grid is spread by size over a batch of uneven groups.
-constexpr int RC_ROWS = 32, RC_WARPS = 8;
+constexpr int RC_ROWS = 32, RC_WARPS = 8, RC_BLOCKS = 4;
+
+// Two blocks run beside a GEMM CTA (crt_overlapped_gemm): both kernels are held to
+// the registers that this leaves them, whatever N is.  Left to itself the compiler
+// took 80 for 15 moduli and more, and one block fitted (2048^3 239 -> 234.5 us,
+// 4000^3 1012 -> 993; at 8000^3, under the power limit, the spread of one side; N = 16
+// .. 18 spill 24 to 80 bytes and take the same time).
+constexpr int regs_at(int threads, int blocks) { return 65536 / (threads * blocks) / 8 * 8; }
+static_assert(C_THREADS * regs_at(C_THREADS, C_BLOCKS) +
+                      2 * 32 * RC_WARPS * regs_at(32 * RC_WARPS, RC_BLOCKS) <= 65536,
+              "a GEMM CTA and two reconstruction blocks share an SM's registers");
 
 __host__ __device__ inline long long recon_items_of(int rows, int cols)
 {
@@ -871,7 +882,7 @@ __device__ __forceinline__ void reconstruct4(const uint32_t (&u4)[N], double *__
 }
 
 template <int N>
-__global__ void __launch_bounds__(32 * RC_WARPS)
+__global__ void __launch_bounds__(32 * RC_WARPS, RC_BLOCKS)
 crt_reconstruct_kernel(const CrtGroup *__restrict__ groups, int g0, int g1, int r0, int r1,
                        long long total, const unsigned char *__restrict__ work)
 {
