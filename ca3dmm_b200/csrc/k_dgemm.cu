@@ -410,12 +410,13 @@ dgemm_dmma_grouped(const CUtensorMap *__restrict__ tmaps, const DProb *__restric
 // Rounding errors grow with the length of a chain of additions, so chunks of
 // 256 k keep the result at least as accurate as the k sub-slabs of up to
 // several thousand k, summed by a kernel of their own, that these shapes ran as
-// before; a segment of more takes one chain more than it must, all of one length.
+// before; the first chain of a longer segment has 128 k, which makes the sum of the
+// squared lengths smaller whatever the rest is.
 // All warps restart at the same block: the additions use the pipe of the
 // MMAs, 1.3 us per chunk of 35 us (0.2 of it the moves to and from TMEM).  With the
 // warps of rows 64 .. 127 half a chunk later they lost 1.8 us, with one m16 tile of
 // a warp at a time, spread over the chunk, 5: an addition waits for the MMAs of the
-// other warp (4736 x 1024 x 8192: 2364, 2427, 2674 us; without restarts 2277, as it is 2345).
+// other warp (4736 x 1024 x 8192: 2364, 2427, 2674 us; without restarts 2277, as it is 2346).
 __device__ __forceinline__ void tmem_ld32_wait(uint32_t taddr, uint32_t (&v)[32])
 {
     asm volatile(
@@ -488,7 +489,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 dgemm_dmma_segments(const __grid_constant__ CUtensorMap map_a,
                     const __grid_constant__ CUtensorMap map_b, const __grid_constant__ DProb prob,
                     const __grid_constant__ SegOrder order,
-                    const ca3dmm_dgemm_seg_t *__restrict__ segs, int split,
+                    const ca3dmm_dgemm_seg_t *__restrict__ segs, int uncut,
                     double2 *__restrict__ partials, int *__restrict__ counters, int *status,
                     unsigned long long limit_ns)
 {
@@ -592,8 +593,11 @@ dgemm_dmma_segments(const __grid_constant__ CUtensorMap map_a,
     for (int pos = first; pos < end && ok; pos += step) {
         const ca3dmm_dgemm_seg_t &sg = segs[pos];
         int left = sg.kt1 - sg.kt0;
-        const int chains = (left + CA3DMM_DGEMM_CHUNK - 1) / CA3DMM_DGEMM_CHUNK + (left >= split);
-        const int chunk = (left + chains - 1) / chains;
+        int chunk = CA3DMM_DGEMM_CHUNK, len = left > chunk ? chunk / 2 : chunk;
+        if (uncut && left > 5) {
+            const int chains = (left + chunk - 1) / chunk + 1;
+            chunk = len = (left + chains - 1) / chains;
+        }
         bool totalled = false;
         for (;;) {
 #pragma unroll
@@ -602,7 +606,8 @@ dgemm_dmma_segments(const __grid_constant__ CUtensorMap map_a,
                 for (int j = 0; j < 4; ++j)
 #pragma unroll
                     for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.0;
-            const int now = min(left, chunk);
+            const int now = min(left, len);
+            len = chunk;
             ok = k_loop<AK, TBN>(smem, full, empty, now, it, acc, &abort_flag, status, limit_ns,
                                  producer, issue_one, wm, wn, g, t, lane);
             if (!ok) break;
@@ -952,8 +957,8 @@ extern "C" int ca3dmm_dgemm_launch_ranges_tn(const void *dev_plan, int nprob,
 // (T = 64, K = 63) 31 blocks against 63: measured 70 us against 148.
 // Products of four rounds or more that equal shares would not shorten by 2 % stay
 // with the grouped kernel (one chain over k, no restarts).  Whole tiles run here
-// with restarts, those of up to one chunk in two chains, as a cut tile has on
-// average: the errors do not grow where the tiles are left whole (1408 x 1408 x 256
+// with restarts, in one chain more than they must and all of one length, as cut tiles
+// have on average: the errors do not grow where the tiles are left whole (1408 x 1408 x 256
 // in one chain 1.86e-16 of |A||B| rms, cut 1.46e-16, in two 1.27e-16; without the
 // restarts long products are 3 to 5 % faster and their errors twice as large).
 // A product of few blocks is not spread over all SMs: the partials read back by
@@ -971,7 +976,6 @@ struct SegShape {
     long long T, K;              // 128 x 128 tiles, 16-k blocks of a tile
     int tiles_m, tiles_n, grid;
     long long whole;             // rounds of whole tiles before the cut ones (-1: nothing is cut)
-    int split;                   // segments of at least so many blocks take one chain more
 };
 
 bool seg_shape(int m, int n, int k, SegShape &s)
@@ -981,7 +985,6 @@ bool seg_shape(int m, int n, int k, SegShape &s)
     s.tiles_n = (n + 127) / 128;
     s.T = (long long) s.tiles_m * s.tiles_n;
     s.K = ((long long) k + BK - 1) / BK;
-    s.split = CA3DMM_DGEMM_CHUNK + 1;
     if (s.T > CA3DMM_DGEMM_SEG_TILES) return false;
     const double dp = (double) ((s.T + SEG_SMS - 1) / SEG_SMS) * (double) s.K;
     double g = std::sqrt(2.5 * (double) s.T * (double) s.T * (double) s.K);
@@ -998,7 +1001,6 @@ bool seg_shape(int m, int n, int k, SegShape &s)
     } else {
         s.whole = -1;
         s.grid = s.T < SEG_SMS ? (int) s.T : SEG_SMS;
-        s.split = 6;
     }
     return true;
 }
@@ -1132,7 +1134,7 @@ extern "C" int ca3dmm_dgemm_segments(int m, int n, int k, int tile_n, ca3dmm_dge
 namespace {
 template <bool AK, int TBN>
 cudaError_t seg_launch_one(int grid, const CUtensorMap *tm, const DProb &prob, const SegOrder &o,
-                           const ca3dmm_dgemm_seg_t *segs, int split, double2 *partials,
+                           const ca3dmm_dgemm_seg_t *segs, int uncut, double2 *partials,
                            int *counters, int *status, unsigned long long limit,
                            cudaStream_t stream)
 {
@@ -1149,7 +1151,7 @@ cudaError_t seg_launch_one(int grid, const CUtensorMap *tm, const DProb &prob, c
         done.fetch_or(bit, std::memory_order_release);
     }
     dgemm_dmma_segments<AK, TBN><<<grid, THREADS, DTile<TBN>::SMEM_BYTES, stream>>>(
-        tm[0], tm[1], prob, o, segs, split, partials, counters, status, limit);
+        tm[0], tm[1], prob, o, segs, uncut, partials, counters, status, limit);
     return cudaGetLastError();
 }
 }  // namespace
@@ -1183,14 +1185,14 @@ extern "C" int ca3dmm_dgemm_launch_segments(const void *host_plan, int nprob,
     double2 *ws = static_cast<double2 *>(partials);
     cudaError_t err;
     if (tile_n == 128)
-        err = a_kmajor ? seg_launch_one<true, 128>(grid, tm, prob, o, dev_segs, s.split, ws, counters,
+        err = a_kmajor ? seg_launch_one<true, 128>(grid, tm, prob, o, dev_segs, s.whole < 0, ws, counters,
                                                     dev_status, limit, stream)
-                       : seg_launch_one<false, 128>(grid, tm, prob, o, dev_segs, s.split, ws, counters,
+                       : seg_launch_one<false, 128>(grid, tm, prob, o, dev_segs, s.whole < 0, ws, counters,
                                                      dev_status, limit, stream);
     else
-        err = a_kmajor ? seg_launch_one<true, 64>(grid, tm, prob, o, dev_segs, s.split, ws, counters,
+        err = a_kmajor ? seg_launch_one<true, 64>(grid, tm, prob, o, dev_segs, s.whole < 0, ws, counters,
                                                    dev_status, limit, stream)
-                       : seg_launch_one<false, 64>(grid, tm, prob, o, dev_segs, s.split, ws, counters,
+                       : seg_launch_one<false, 64>(grid, tm, prob, o, dev_segs, s.whole < 0, ws, counters,
                                                     dev_status, limit, stream);
     CA3DMM_CUDA_TRY(err);
     ca3dmm_note_launch(1);
