@@ -988,7 +988,7 @@ static void a_pack_desc(const ca3dmm_engine_p e, const plan_t *pl, const blk_t *
 
 /* Build the per-call device plan into pinned staging and upload it. */
 static int plan_upload(ca3dmm_engine_p e, const void *A, int ldA, const void *B, int ldB,
-                       void *dst, int ldC, cudaStream_t st)
+                       void *dst, int ldC, int sync, cudaStream_t st)
 {
     plan_t *pl = (plan_t *) e->impl;
     int rc = ca3dmm_stage_begin(&pl->stage);
@@ -1256,7 +1256,7 @@ static int plan_upload(ca3dmm_engine_p e, const void *A, int ldA, const void *B,
         e->crt_bits = pl->crt.p_min;
     }
     memset(h + pl->off_counters, 0, COUNTER_BYTES);
-    rc = ca3dmm_stage_upload(&pl->stage, w, st);
+    rc = ca3dmm_stage_upload(&pl->stage, w, sync, st);
     if (rc) return rc;
     for (int i = 0; i < pl->ncanary; i++)
         CA3DMM_CUDA_TRY(cudaMemsetAsync(w + pl->canary[i], CANARY_BYTE, CANARY_BYTES, st));
@@ -1426,7 +1426,7 @@ static int exec_device(ca3dmm_engine_p e, const void *src_A, int ldA, const void
     int rc;
     if (!pl->plan_valid || pl->c_A != src_A || pl->c_B != src_B || pl->c_ldA != ldA ||
         pl->c_ldB != ldB || pl->c_dst != dst_C || pl->c_ldC != ldC) {
-        rc = plan_upload(e, src_A, ldA, src_B, ldB, dst_C, ldC, st);
+        rc = plan_upload(e, src_A, ldA, src_B, ldB, dst_C, ldC, e->sync_exec, st);
         if (rc) return rc;
     } else {
         rc = counters_clear(pl, w, e->sync_exec, st);
@@ -1520,6 +1520,7 @@ static int exec_device(ca3dmm_engine_p e, const void *src_A, int ldA, const void
     if (rc) return rc;
     if (e->sync_exec) {
         CA3DMM_CUDA_TRY(cudaStreamSynchronize(st));
+        ca3dmm_stage_done(&pl->stage);
         rc = device_status_error(pl);
         if (rc) return rc;
         pl->counters_clean = 1;
@@ -1975,7 +1976,7 @@ static int exec_host(ca3dmm_engine_p e, const void *A_h, int ldA, const void *B_
     if (!pl->plan_valid || pl->c_A != dAsrc || pl->c_B != x->dB || pl->c_ldA != ldAsrc ||
         pl->c_ldB != x->ldb || pl->c_dst != x->dC || pl->c_ldC != x->ldc) {
         pl->upload_for_host = 1;
-        rc = plan_upload(e, dAsrc, (int) ldAsrc, x->dB, (int) x->ldb, x->dC, (int) x->ldc, st);
+        rc = plan_upload(e, dAsrc, (int) ldAsrc, x->dB, (int) x->ldb, x->dC, (int) x->ldc, 1, st);
         pl->upload_for_host = 0;
         if (rc) return rc;
         x->built_mode = -1;
@@ -1986,6 +1987,7 @@ static int exec_host(ca3dmm_engine_p e, const void *A_h, int ldA, const void *B_
         hx_build_bands(e, x, st);
     /* the inputs may not be overwritten before the previous exec's reads are done */
     CA3DMM_CUDA_TRY(cudaStreamSynchronize(st));
+    ca3dmm_stage_done(&pl->stage);
     if (e->is_BTB) {
         const int r = hx_btb_slabs(e, x, B_h, ldB, C_h, ldC, st);
         if (r != 1) return r;

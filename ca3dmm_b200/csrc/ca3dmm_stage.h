@@ -13,7 +13,8 @@ typedef struct {
     void *buf;
     size_t bytes;
     cudaEvent_t done;      /* recorded behind the last upload */
-    int pending;           /* that upload may not have run yet */
+    int pending;           /* the last upload may not have run yet: 1 until `done`, 2 until the
+                              call that queued it has waited for its stream */
     int in_graph;          /* a graph reads buf */
     int any_graph;         /* some graph may overwrite the device plan at any time */
     void **kept;           /* the buffers of captured uploads, held until the owner goes */
@@ -62,32 +63,38 @@ static inline int ca3dmm_stage_begin(ca3dmm_stage_t *s)
             s->buf = nb;
             s->in_graph = 0;
         }
-    } else if (cudaEventSynchronize(s->done) != cudaSuccess) {
-        rc = CA3DMM_ECUDA;
+    } else if ((s->pending == 1 ? cudaEventSynchronize(s->done) : cudaDeviceSynchronize()) !=
+               cudaSuccess) {
+        rc = CA3DMM_ECUDA;                /* (2: that call failed before its wait) */
     }
     if (!rc) s->pending = 0;
     cudaThreadExchangeStreamCaptureMode(&mode);
     return rc;
 }
 
-/* Queue the copy of buf.  Afterwards any_graph says whether the device copy can
+/* Queue the copy of buf; sync: the caller waits for the stream before it returns and
+ * then calls ca3dmm_stage_done, which spares the event (3 us a call).  Afterwards any_graph says whether the device copy can
  * be relied on by a later call: one that waits in a graph has not run yet, and
  * each replay puts that graph's plan back. */
-static inline int ca3dmm_stage_upload(ca3dmm_stage_t *s, void *dst, cudaStream_t st)
+static inline int ca3dmm_stage_upload(ca3dmm_stage_t *s, void *dst, int sync, cudaStream_t st)
 {
     enum cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
+    if (!sync && cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
         cudaGetLastError();              /* the legacy stream beside another thread's capture */
         cap = cudaStreamCaptureStatusNone;
     }
     CA3DMM_CUDA_TRY(cudaMemcpyAsync(dst, s->buf, s->bytes, cudaMemcpyHostToDevice, st));
     if (cap == cudaStreamCaptureStatusActive) {
         s->in_graph = s->any_graph = 1;
+    } else if (sync) {
+        s->pending = 2;
     } else {
         CA3DMM_CUDA_TRY(cudaEventRecord(s->done, st));
         s->pending = 1;
     }
     return CA3DMM_OK;
 }
+
+static inline void ca3dmm_stage_done(ca3dmm_stage_t *s) { s->pending = 0; }
 
 #endif

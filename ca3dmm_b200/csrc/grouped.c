@@ -340,7 +340,7 @@ static int build_plan(ca3dmm_grouped_p g, const double *const *A, const int *ldA
         }
         if (rc) return rc;
     }
-    rc = ca3dmm_stage_upload(&g->stage, w, st);
+    rc = ca3dmm_stage_upload(&g->stage, w, g->sync, st);
     if (rc) return rc;
     for (int i = 0; i < np; i++) {
         g->cA[i] = A[i]; g->cB[i] = B[i]; g->cC[i] = C[i];
@@ -402,6 +402,7 @@ int ca3dmm_grouped_exec(ca3dmm_grouped_p g, const double *const *A, const int *l
     if (g->sync) {
         CA3DMM_CUDA_TRY(cudaMemcpyAsync(g->status_h, status, sizeof(int), cudaMemcpyDeviceToHost, st));
         CA3DMM_CUDA_TRY(cudaStreamSynchronize(st));
+        ca3dmm_stage_done(&g->stage);
         if (g->status_h[0]) {
             ERROR_PRINTF("grouped GEMM: device status %d (a bounded wait ran out)\n", g->status_h[0]);
             return CA3DMM_ETIMEOUT;

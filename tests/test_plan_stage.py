@@ -28,6 +28,7 @@ cudaError_t cudaThreadExchangeStreamCaptureMode(enum cudaStreamCaptureMode *);
 cudaError_t cudaStreamIsCapturing(cudaStream_t, enum cudaStreamCaptureStatus *);
 cudaError_t cudaMemcpyAsync(void *, const void *, size_t, int, cudaStream_t);
 cudaError_t cudaGetLastError(void);
+cudaError_t cudaDeviceSynchronize(void);
 #endif
 """
 
@@ -85,12 +86,20 @@ cudaError_t cudaMemcpyAsync(void *d, const void *src, size_t n, int k, cudaStrea
 }
 cudaError_t cudaGetLastError(void) { return 0; }
 
-static int plan(ca3dmm_stage_t *s, int value, int *dev)
+cudaError_t cudaDeviceSynchronize(void)
+{
+    if (capturing && mode != cudaStreamCaptureModeRelaxed) return 1;
+    run_queue(nq);
+    return 0;
+}
+
+static int plan_of(ca3dmm_stage_t *s, int value, int *dev, int sync)
 {
     if (ca3dmm_stage_begin(s)) return 1;
     *(int *) s->buf = value;
-    return ca3dmm_stage_upload(s, dev, 0);
+    return ca3dmm_stage_upload(s, dev, sync, 0);
 }
+static int plan(ca3dmm_stage_t *s, int value, int *dev) { return plan_of(s, value, dev, 0); }
 #define CHECK(x) do { if (!(x)) { printf("line %d: %s\n", __LINE__, #x); return 1; } } while (0)
 
 int main(void)
@@ -120,6 +129,14 @@ int main(void)
         for (int i = 0; i < ng; i++) *graph[i].dst = *graph[i].src;
     CHECK(dev[3] == 20 && dev[4] == 21 && dev[5] == 22 && dev[6] == 23 && dev[7] == 24);
     CHECK(mode == cudaStreamCaptureModeGlobal);
+    /* synchronous calls: one that waited for its stream, one that failed before it did */
+    CHECK(plan_of(&s, 30, &dev[0], 1) == 0);
+    run_queue(nq);
+    ca3dmm_stage_done(&s);
+    CHECK(plan_of(&s, 31, &dev[1], 1) == 0);
+    CHECK(plan(&s, 32, &dev[2]) == 0);
+    run_queue(nq);
+    CHECK(dev[0] == 30 && dev[1] == 31 && dev[2] == 32);
     ca3dmm_stage_free(&s);
     CHECK(live == 0);
     return 0;
