@@ -509,9 +509,10 @@ extern "C" int ca3dmm_copy_runs_launch(const ca3dmm_run_piece_t *pieces, int n, 
 {
     if (n < 0 || n > CA3DMM_MAX_RUN_PIECES) return CA3DMM_EINVAL;
     if (n == 0) return CA3DMM_OK;
-    // two parameter sizes: small launches carry less
-    CA3DMM_CUDA_TRY(n <= 64 ? copy_runs_launch<64>(pieces, n, stream)
-                            : copy_runs_launch<CA3DMM_MAX_RUN_PIECES>(pieces, n, stream));
+    // the launch copies its parameters (24 KB at 512 blocks, 2 us): as few as hold them
+    CA3DMM_CUDA_TRY(n <= 32    ? copy_runs_launch<32>(pieces, n, stream)
+                    : n <= 128 ? copy_runs_launch<128>(pieces, n, stream)
+                               : copy_runs_launch<CA3DMM_MAX_RUN_PIECES>(pieces, n, stream));
     return CA3DMM_OK;
 }
 
