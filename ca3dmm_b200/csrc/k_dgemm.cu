@@ -410,8 +410,8 @@ dgemm_dmma_grouped(const CUtensorMap *__restrict__ tmaps, const DProb *__restric
 // Rounding errors grow with the length of a chain of additions, so chunks of
 // 256 k keep the result at least as accurate as the k sub-slabs of up to
 // several thousand k, summed by a kernel of their own, that these shapes ran as
-// before; the first chain of a longer segment has 128 k, which makes the sum of the
-// squared lengths smaller whatever the rest is.
+// before; the last chain but one of a longer segment has 128 k, which makes the sum of
+// the squared lengths smaller whatever the rest is.
 // All warps restart at the same block: the additions use the pipe of the
 // MMAs, 1.3 us per chunk of 35 us (0.2 of it the moves to and from TMEM).  With the
 // warps of rows 64 .. 127 half a chunk later they lost 1.8 us, with one m16 tile of
@@ -593,10 +593,11 @@ dgemm_dmma_segments(const __grid_constant__ CUtensorMap map_a,
     for (int pos = first; pos < end && ok; pos += step) {
         const ca3dmm_dgemm_seg_t &sg = segs[pos];
         int left = sg.kt1 - sg.kt0;
-        int chunk = CA3DMM_DGEMM_CHUNK, len = left > chunk ? chunk / 2 : chunk;
+        int chunk = CA3DMM_DGEMM_CHUNK;
+        bool half = !uncut && left > chunk;          // the chain of half a chunk is to come
         if (uncut && left > 5) {
             const int chains = (left + chunk - 1) / chunk + 1;
-            chunk = len = (left + chains - 1) / chains;
+            chunk = (left + chains - 1) / chains;
         }
         bool totalled = false;
         for (;;) {
@@ -606,8 +607,11 @@ dgemm_dmma_segments(const __grid_constant__ CUtensorMap map_a,
                 for (int j = 0; j < 4; ++j)
 #pragma unroll
                     for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.0;
-            const int now = min(left, len);
-            len = chunk;
+            int now = min(left, chunk);
+            if (half && left <= chunk + chunk / 2) {
+                now = chunk / 2;
+                half = false;
+            }
             ok = k_loop<AK, TBN>(smem, full, empty, now, it, acc, &abort_flag, status, limit_ns,
                                  producer, issue_one, wm, wn, g, t, lane);
             if (!ok) break;
