@@ -594,10 +594,11 @@ dgemm_dmma_segments(const __grid_constant__ CUtensorMap map_a,
         const ca3dmm_dgemm_seg_t &sg = segs[pos];
         int left = sg.kt1 - sg.kt0;
         int chunk = CA3DMM_DGEMM_CHUNK;
-        bool half = !uncut && left > chunk;          // the chain of half a chunk is to come
-        if (uncut && left > 5) {
+        bool half = left > chunk;                    // the chain of half a chunk is to come
+        if (uncut && left > 5 && left < 4 * chunk) {
             const int chains = (left + chunk - 1) / chunk + 1;
             chunk = (left + chains - 1) / chains;
+            half = false;
         }
         bool totalled = false;
         for (;;) {
@@ -961,8 +962,8 @@ extern "C" int ca3dmm_dgemm_launch_ranges_tn(const void *dev_plan, int nprob,
 // (T = 64, K = 63) 31 blocks against 63: measured 70 us against 148.
 // Products of four rounds or more that equal shares would not shorten by 2 % stay
 // with the grouped kernel (one chain over k, no restarts).  Whole tiles run here
-// with restarts, in one chain more than they must and all of one length, as cut tiles
-// have on average: the errors do not grow where the tiles are left whole (1408 x 1408 x 256
+// with restarts, those of less than 1024 k in one chain more than they must and all of one
+// length, as cut tiles have on average: the errors do not grow where the tiles are left whole (1408 x 1408 x 256
 // in one chain 1.86e-16 of |A||B| rms, cut 1.46e-16, in two 1.27e-16; without the
 // restarts long products are 3 to 5 % faster and their errors twice as large).
 // A product of few blocks is not spread over all SMs: the partials read back by
