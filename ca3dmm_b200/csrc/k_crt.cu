@@ -638,8 +638,8 @@ crt_gemm_kernel(const CrtGroup *__restrict__ groups, int ngroup, int nmod,
             // at an offset known when it is compiled.  (With one byte stored at a time and
             // eight instructions per sum, 256 uneven products took 4.47 ms of GEMM, with
             // this 4.28, with items decoded ahead 4.0; the 8000^3 product 4.92, 4.83 ms.)
-            // columns past tile_cols were not accumulated (still zero) and lie
-            // past the group's n (never read): skipped
+            // columns past tile_cols were not accumulated (still at their start) and
+            // lie past the group's n (never read): skipped
 #pragma unroll 1
             for (int cb = 0; cb < TN / 64; ++cb) {
                 const int c0 = h * (TN / 2) + cb * 32;

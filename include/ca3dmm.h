@@ -229,7 +229,8 @@ void ca3dmm_engine_set_stream(ca3dmm_engine_p engine, void *stream, int sync);
  * *workbuf_bytes, which ca3dmm_engine_workbuf_bytes reports). */
 int ca3dmm_engine_set_gemm_mode(ca3dmm_engine_p engine, int mode, int slices);
 size_t ca3dmm_engine_workbuf_bytes(ca3dmm_engine_p engine);
-/* Tile rows per raster band of the GEMM launches (4, 8 or 16; L2 reuse). */
+/* Tile rows per raster band of the GEMM launches (4, 8 or 16; L2 reuse).  Plain
+ * products that run as k segments (C of few tiles) keep bands of 8. */
 int ca3dmm_engine_set_raster(ca3dmm_engine_p engine, int raster);
 /* Geometry of any virtual rank, same 34-int layout as the CPU oracle's
  * orc_rank_geometry: is_active, rank_m/n/k, task_{m,n,k}_{num,id},
