@@ -959,7 +959,7 @@ extern "C" int ca3dmm_dgemm_launch_ranges_tn(const void *dev_plan, int nprob,
 // tiles): fitted to 530 shapes of 1 to 2368 tiles and 2 to 1024 blocks, where the
 // choice is within 7 % of the better one and 0.06 % on average (with 1.9 in place of
 // 2 to 7 it lost up to 16 %, 1408 x 1408 x 256 took 78 us and now takes 68).  At 1000^3
-// (T = 64, K = 63) 31 blocks against 63: measured 70 us against 148.
+// (T = 64, K = 63) 31 blocks against 63: a call takes 101 us, 194 in whole tiles.
 // Products of four rounds or more that equal shares would not shorten by 2 % stay
 // with the grouped kernel (one chain over k, no restarts).  Whole tiles run here
 // with restarts, those of less than 1024 k in one chain more than they must and all of one

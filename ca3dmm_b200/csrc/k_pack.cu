@@ -265,7 +265,7 @@ copy_block_kernel(const double *__restrict__ src, long long lds, double *__restr
 // 8000 x 8000 from 24 column strips to 4 x 6 blocks (116 pieces, 1.02 GB): 178 us,
 // 5.75 TB/s (one piece after the other 199-214; with default loads and stores in
 // place of the streaming ones, lines aligned, 373; 64 x 64 tiles from descriptors
-// in memory 206).  The call: 242 -> 206 us, with the upload of the descriptors and
+// in memory 206).  The call: 241 -> 206 us, with the upload of the descriptors and
 // the wait before it gone.
 // Runs of up to RUN_NARROW elements are too short for that: two of them in flight are
 // less than the memory's latency asks for.  An item takes as many as fill 64 loads of

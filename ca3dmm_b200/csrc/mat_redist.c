@@ -142,6 +142,8 @@ struct mat_redist_layouts {
     int by_value;                 /* few enough pieces to travel with the launch */
     ca3dmm_pack_desc_t *desc_h;   /* pinned staging of the descriptors */
     ca3dmm_pack_desc_t *desc_d;
+    cudaEvent_t done;             /* recorded behind the copy that reads them */
+    int pending;
 };
 
 int mat_redist_layouts_init(int nsrc, const int *src_rects, int nreq, const int *req_rects,
@@ -191,7 +193,8 @@ int mat_redist_layouts_init(int nsrc, const int *src_rects, int nreq, const int 
         const size_t bytes = sizeof(ca3dmm_pack_desc_t) * (size_t) L->npiece;
         if (cudaMallocHost((void **) &L->desc_h, bytes) != cudaSuccess) L->desc_h = NULL;
         if (cudaMalloc((void **) &L->desc_d, bytes) != cudaSuccess) L->desc_d = NULL;
-        if (!L->desc_h || !L->desc_d) {
+        if (!L->desc_h || !L->desc_d ||
+            cudaEventCreateWithFlags(&L->done, cudaEventDisableTiming) != cudaSuccess) {
             mat_redist_layouts_free(&L);
             return CA3DMM_ENOMEM;
         }
@@ -233,8 +236,11 @@ int mat_redist_layouts_exec(mat_redist_layouts_p L, const void *const *src_blks,
         if (!stream) CA3DMM_CUDA_TRY(cudaStreamSynchronize(st));
         return CA3DMM_OK;
     }
-    /* the staging is rewritten below: the previous exec's upload must be done */
+    /* the descriptors are rewritten below: the previous exec, on this stream or another,
+     * must be through with them */
     CA3DMM_CUDA_TRY(cudaStreamSynchronize(st));
+    if (L->pending) CA3DMM_CUDA_TRY(cudaEventSynchronize(L->done));
+    L->pending = 0;
     for (int k = 0; k < L->npiece; k++) {
         const piece_t *p = &L->pieces[k];
         const int *s = L->src_rects + 4 * p->src, *r = L->req_rects + 4 * p->dst;
@@ -255,6 +261,8 @@ int mat_redist_layouts_exec(mat_redist_layouts_p L, const void *const *src_blks,
     CA3DMM_CUDA_TRY(cudaMemcpyAsync(L->desc_d, L->desc_h, sizeof(ca3dmm_pack_desc_t) * L->npiece,
                                     cudaMemcpyHostToDevice, st));
     int rc = ca3dmm_pack_launch(NULL, NULL, L->desc_d, L->npiece, tiles, st);
+    CA3DMM_CUDA_TRY(cudaEventRecord(L->done, st));
+    L->pending = 1;
     if (rc) return rc;
     if (!stream) CA3DMM_CUDA_TRY(cudaStreamSynchronize(st));
     return CA3DMM_OK;
@@ -269,6 +277,7 @@ void mat_redist_layouts_free(mat_redist_layouts_p *Lp)
     free(L->pieces);
     if (L->desc_h) cudaFreeHost(L->desc_h);
     if (L->desc_d) cudaFree(L->desc_d);
+    if (L->done) cudaEventDestroy(L->done);
     free(L);
     *Lp = NULL;
 }

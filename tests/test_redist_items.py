@@ -127,3 +127,30 @@ def test_longest_runs(cuda, length):
     del src, dst
     torch.cuda.empty_cache()
     assert same
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("strips,pr,pc", [(64, 9, 10), (7, 3, 2)])    # more than 512 pieces, fewer
+def test_two_streams(cuda, strips, pr, pc):
+    """One handle on two streams, the first held up: each exec moves its own blocks."""
+    import torch
+    n = 640
+    cut = lambda p: [(n * i // p, n * (i + 1) // p - n * i // p) for i in range(p)]
+    src = [(0, c0, n, w) for c0, w in cut(strips)]
+    dst = [(r0, c0, h, w) for r0, h in cut(pr) for c0, w in cut(pc)]
+    lay = cb.RedistLayouts(src, dst)
+    assert lay.ok
+    sets = []
+    for _ in range(2):
+        G = torch.rand(n, n, dtype=torch.float64, device="cuda")
+        blocks = lambda R: [G[r:r + h, c:c + w].contiguous() for r, c, h, w in R]
+        S, want = blocks(src), blocks(dst)
+        sets.append((S, [torch.zeros_like(w) for w in want], want, torch.cuda.Stream()))
+    torch.cuda.synchronize()
+    with torch.cuda.stream(sets[0][3]):
+        torch.cuda._sleep(20_000_000)
+    for S, D, _, s in sets:
+        assert lay.exec(S, [x.shape[1] for x in S], D, [x.shape[1] for x in D], s.cuda_stream) == 0
+    torch.cuda.synchronize()
+    for _, D, want, _ in sets:
+        assert all(torch.equal(a, b) for a, b in zip(D, want))
