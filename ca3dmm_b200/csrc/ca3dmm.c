@@ -1763,8 +1763,8 @@ static int hx_build_bands(ca3dmm_engine_p e, struct host_exec *x, cudaStream_t s
             char *dh = (char *) x->desc_h + (size_t) c * x->desc_stride;
             for (int tk = 0; tk < e->kp; tk++) blocks[tk] = tk * tmn + tm;
             if (ozaki) {
-                bad = ca3dmm_oz_encode_rows((char *) pl->stage.buf + pl->off_ozplan, pl->ngroup, blocks,
-                                            e->kp, r, rend, dh, x->ntile[c]);
+                bad = ca3dmm_oz_encode_rows((char *) pl->stage.buf + pl->off_ozplan, pl->ngroup,
+                                            blocks, e->kp, r, rend, dh, x->ntile[c]);
             } else {
                 ca3dmm_pack_desc_t *pd = (ca3dmm_pack_desc_t *) dh;
                 for (int tk = 0; tk < e->kp; tk++) {
@@ -1901,8 +1901,8 @@ static int hx_btb_slabs(ca3dmm_engine_p e, struct host_exec *x, const void *B_h,
         if (crt) {
             const void *dd = (const char *) x->desc_d + (size_t) j * x->desc_stride;
             int ib = 0, ic = 0;
-            rc = ca3dmm_crt_group_items((char *) pl->stage.buf + pl->off_crtplan, j, 0, INT32_MAX, &ib,
-                                        &ic);
+            rc = ca3dmm_crt_group_items((char *) pl->stage.buf + pl->off_crtplan, j, 0, INT32_MAX,
+                                        &ib, &ic);
             rg.begin[0] = ib;
             rg.len[0] = ic;
             if (!rc) rc = ca3dmm_crt_pack_descs(&pl->crt, x->dB, dd, 1, x->ntile[j], st);

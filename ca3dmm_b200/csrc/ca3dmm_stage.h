@@ -73,9 +73,9 @@ static inline int ca3dmm_stage_begin(ca3dmm_stage_t *s)
 }
 
 /* Queue the copy of buf; sync: the caller waits for the stream before it returns and
- * then calls ca3dmm_stage_done, which spares the event (3 us a call).  Afterwards any_graph says whether the device copy can
- * be relied on by a later call: one that waits in a graph has not run yet, and
- * each replay puts that graph's plan back. */
+ * then calls ca3dmm_stage_done, which spares the event (3 us a call).  Afterwards
+ * any_graph says whether the device copy can be relied on by a later call: one that
+ * waits in a graph has not run yet, and each replay puts that graph's plan back. */
 static inline int ca3dmm_stage_upload(ca3dmm_stage_t *s, void *dst, int sync, cudaStream_t st)
 {
     enum cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;

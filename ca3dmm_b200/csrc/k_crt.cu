@@ -62,7 +62,7 @@ struct CrtTile {
     static constexpr size_t kSmem = (size_t) kStages * kStageBytes + (2 * kStages + 4) * 8 + 1024;
 };
 constexpr int C_THREADS = 384;                   // 12 warps
-constexpr int C_BLOCKS = 2;                      // its registers: half an SM's (shared memory holds one)
+constexpr int C_BLOCKS = 2;                      // holds it to half an SM's registers
 constexpr int C_ISSUERS = 2;
 constexpr int C_EPI_WARPS = 8;
 constexpr int GROUP_CACHE = 512;
@@ -486,8 +486,8 @@ crt_gemm_kernel(const CrtGroup *__restrict__ groups, int ngroup, int nmod,
             uint32_t it = 0, ii = 0;
             bool ok = true;
             for (int v = blockIdx.x; v < total_items && ok && !abort_flag; v += gridDim.x) {
-                if (!mbar_wait_bounded(&item_full[ii % ITEM_RING], (ii / ITEM_RING) & 1u, &abort_flag,
-                                       status, CA3DMM_DEV_TIMEOUT_PRODUCE, limit_ns))
+                if (!mbar_wait_bounded(&item_full[ii % ITEM_RING], (ii / ITEM_RING) & 1u,
+                                       &abort_flag, status, CA3DMM_DEV_TIMEOUT_PRODUCE, limit_ns))
                     break;
                 const CrtItem &I = ring[ii % ITEM_RING];
                 const unsigned char *qa = I.qa, *qb = I.qb;
@@ -523,8 +523,8 @@ crt_gemm_kernel(const CrtGroup *__restrict__ groups, int ngroup, int nmod,
             uint32_t it = 0, ai = 0;
             bool ok = true;
             for (int v = blockIdx.x; v < total_items && ok; v += gridDim.x, ++ai) {
-                if (!mbar_wait_bounded(&item_full[ai % ITEM_RING], (ai / ITEM_RING) & 1u, &abort_flag,
-                                       status, CA3DMM_DEV_TIMEOUT_ACCUM, limit_ns)) {
+                if (!mbar_wait_bounded(&item_full[ai % ITEM_RING], (ai / ITEM_RING) & 1u,
+                                       &abort_flag, status, CA3DMM_DEV_TIMEOUT_ACCUM, limit_ns)) {
                     ok = false;
                     break;
                 }

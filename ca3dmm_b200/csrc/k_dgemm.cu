@@ -416,7 +416,7 @@ dgemm_dmma_grouped(const CUtensorMap *__restrict__ tmaps, const DProb *__restric
 // MMAs, 1.3 us per chunk of 35 us (0.2 of it the moves to and from TMEM).  With the
 // warps of rows 64 .. 127 half a chunk later they lost 1.8 us, with one m16 tile of
 // a warp at a time, spread over the chunk, 5: an addition waits for the MMAs of the
-// other warp (4736 x 1024 x 8192: 2364, 2427, 2674 us; without restarts 2277, as it is 2346).
+// other warp (4736 x 1024 x 8192: 2364, 2427, 2674 us; without restarts 2277).
 __device__ __forceinline__ void tmem_ld32_wait(uint32_t taddr, uint32_t (&v)[32])
 {
     asm volatile(
@@ -962,10 +962,11 @@ extern "C" int ca3dmm_dgemm_launch_ranges_tn(const void *dev_plan, int nprob,
 // (T = 64, K = 63) 31 blocks against 63: a call takes 101 us, 194 in whole tiles.
 // Products of four rounds or more that equal shares would not shorten by 2 % stay
 // with the grouped kernel (one chain over k, no restarts).  Whole tiles run here
-// with restarts, those of less than 1024 k in one chain more than they must and all of one
-// length, as cut tiles have on average: the errors do not grow where the tiles are left whole (1408 x 1408 x 256
-// in one chain 1.86e-16 of |A||B| rms, cut 1.46e-16, in two 1.27e-16; without the
-// restarts long products are 3 to 5 % faster and their errors twice as large).
+// with restarts, those of less than 1024 k in one chain more than they must and all
+// of one length, as cut tiles have on average: the errors do not grow where the
+// tiles are left whole (1408 x 1408 x 256 in one chain 1.87e-16 of |A||B| rms, cut
+// 1.47e-16, in two 1.34e-16; without the restarts long products are 3 to 5 % faster
+// and their errors twice as large).
 // A product of few blocks is not spread over all SMs: the partials read back by
 // the last CTA of a tile grow with the parts, so the number of CTAs is at most
 // sqrt(2.5 T T K).  From k = 512 on a share is at least one chunk: chains of 256 k
@@ -1188,17 +1189,18 @@ extern "C" int ca3dmm_dgemm_launch_segments(const void *host_plan, int nprob,
     if (!seg_shape(prob.m, prob.n, prob.k, s)) return CA3DMM_EINVAL;
     const unsigned long long limit = (unsigned long long) (timeout_s * 1e9);
     double2 *ws = static_cast<double2 *>(partials);
+    const int uncut = s.whole < 0;
     cudaError_t err;
     if (tile_n == 128)
-        err = a_kmajor ? seg_launch_one<true, 128>(grid, tm, prob, o, dev_segs, s.whole < 0, ws, counters,
-                                                    dev_status, limit, stream)
-                       : seg_launch_one<false, 128>(grid, tm, prob, o, dev_segs, s.whole < 0, ws, counters,
-                                                     dev_status, limit, stream);
-    else
-        err = a_kmajor ? seg_launch_one<true, 64>(grid, tm, prob, o, dev_segs, s.whole < 0, ws, counters,
+        err = a_kmajor ? seg_launch_one<true, 128>(grid, tm, prob, o, dev_segs, uncut, ws, counters,
                                                    dev_status, limit, stream)
-                       : seg_launch_one<false, 64>(grid, tm, prob, o, dev_segs, s.whole < 0, ws, counters,
+                       : seg_launch_one<false, 128>(grid, tm, prob, o, dev_segs, uncut, ws, counters,
                                                     dev_status, limit, stream);
+    else
+        err = a_kmajor ? seg_launch_one<true, 64>(grid, tm, prob, o, dev_segs, uncut, ws, counters,
+                                                  dev_status, limit, stream)
+                       : seg_launch_one<false, 64>(grid, tm, prob, o, dev_segs, uncut, ws, counters,
+                                                   dev_status, limit, stream);
     CA3DMM_CUDA_TRY(err);
     ca3dmm_note_launch(1);
     return CA3DMM_OK;

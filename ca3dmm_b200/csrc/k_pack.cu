@@ -16,7 +16,8 @@
 namespace {
 
 constexpr int PT = 64;   // pack tile edge
-__host__ __device__ constexpr int pack_tiles_of(int n) { return (n - 1) / PT + 1; }   // n + 63 may not fit
+// (n + 63 may not fit)
+__host__ __device__ constexpr int pack_tiles_of(int n) { return (n - 1) / PT + 1; }
 
 __device__ __forceinline__ int find_desc(const ca3dmm_pack_desc_t *d, int n, int tile)
 {
@@ -280,7 +281,10 @@ constexpr int RUN_E = 512, RUN_GROUP = 4, RUN_NARROW = 128, RUN_LOADS = 32;
 __host__ __device__ inline bool run_narrow(int len) { return len <= RUN_NARROW; }
 // narrow: loads per run, and log2 of the lanes that share one
 __host__ __device__ inline int run_loads(int len) { return len <= 32 ? 1 : len <= 64 ? 2 : 4; }
-__host__ __device__ inline int run_lanes(int len) { return len > 16 ? 5 : len > 8 ? 4 : len > 4 ? 3 : len > 2 ? 2 : len > 1 ? 1 : 0; }
+__host__ __device__ inline int run_lanes(int len)
+{
+    return len > 16 ? 5 : len > 8 ? 4 : len > 4 ? 3 : len > 2 ? 2 : len > 1 ? 1 : 0;
+}
 inline int run_chunks(int len) { return run_narrow(len) ? 1 : (len + 15 + RUN_E - 1) / RUN_E; }
 inline int run_group(int len)
 {
@@ -291,7 +295,7 @@ struct RunPiece {
     const double *src;
     double *dst;
     int lds, ldd, len, runs;
-    int begin, nch, group;               // first item (blocks one after the other), chunks, runs per item
+    int begin, nch, group;           // first item (blocks one after the other), chunks, runs per item
 };
 
 template <int CAP>
@@ -300,7 +304,7 @@ struct RunPieces {
 };
 
 struct RunItems {
-    int npiece, turn, total;                         // turn: chunks per block in turn (0: one after the other)
+    int npiece, turn, total;         // turn: chunks per block in turn (0: one after the other)
 };
 
 struct RunItem {
@@ -463,7 +467,8 @@ extern "C" long long ca3dmm_copy_runs_items(const ca3dmm_run_piece_t *pieces, in
                ? (long long) wide.total + narrow.total : -1;
 }
 
-extern "C" int ca3dmm_copy_runs_item(const ca3dmm_run_piece_t *pieces, int n, long long item, int *out5)
+extern "C" int ca3dmm_copy_runs_item(const ca3dmm_run_piece_t *pieces, int n, long long item,
+                                     int *out5)
 {
     RunPieces<CA3DMM_MAX_RUN_PIECES> P;
     RunItems I;
@@ -474,11 +479,10 @@ extern "C" int ca3dmm_copy_runs_item(const ca3dmm_run_piece_t *pieces, int n, lo
     const RunItem w = run_item(P.p, I, (int) item);
     const RunPiece &d = P.p[w.piece];
     out5[0] = 0;
-    for (int i = 0, of = 0; of < w.piece || run_narrow(pieces[i].len) != narrow || pieces[i].len <= 0 ||
-                            pieces[i].runs <= 0; ++i) {
+    for (int i = 0, of = 0;; ++i) {
         if (pieces[i].len <= 0 || pieces[i].runs <= 0) continue;
+        if (run_narrow(pieces[i].len) == narrow && of++ == w.piece) break;
         ++out5[0];
-        if (run_narrow(pieces[i].len) == narrow) ++of;
     }
     out5[1] = w.run0;
     out5[2] = w.run1;
